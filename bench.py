@@ -43,7 +43,7 @@ SEED = 2024
 
 # FP32 operations of one in-cutoff pair of the full evaluation (u, du_dx,
 # du_dp, du_dl), counted on the per-pair arithmetic of the pair kernel
-# (timemachine_b200/csrc/nb_pair_math.cuh, pair_terms / sweep_tile in
+# (timemachine_b200/csrc/nb_pair_math.cuh, walk_pairs in
 # nb_kernels.cuh), which restates timemachine/cpp/src/kernels/nonbonded_common.cuh:38-140
 # and k_nonbonded.cuh:424-512. FMA = 2; FMUL, FADD = 1; rsqrt, ex2 and the
 # IEEE reciprocal = 1 each; the fixed-point scalings (v * 2^e) are counted,

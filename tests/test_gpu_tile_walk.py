@@ -1,0 +1,91 @@
+"""The tile walk of the pair kernel against the pair-list kernel over the same
+pairs: every output is an exact integer sum of per-pair fixed-point values, and
+both kernels round a pair the same way, so they agree bit for bit. Sizes sit at
+the edges of tiles and row groups; coordinates lie in several periodic images
+(one-image shift and general minimum image); random positions bring pairs whose
+terms exceed the shared-memory limbs; a dense group fills the list builder's
+column buffer."""
+
+import numpy as np
+import pytest
+
+from tests.helpers import f32_round, random_params
+from timemachine_b200 import potentials as P
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(n, seed, images):
+    rng = np.random.default_rng(seed)
+    edges = np.array([3.1, 3.4, 5.3])
+    x = rng.uniform(0, 1, size=(n, 3)) * edges
+    x = x + rng.integers(-images, images + 1, size=(n, 3)) * edges
+    params = random_params(rng, n)
+    params[rng.random(n) < 0.6, 2] = 0.0  # most atoms without Lennard-Jones terms, as in water
+    plane = rng.integers(-1, 2, size=n).astype(np.int32) * (rng.random(n) < 0.1)
+    offset = rng.integers(-1, 2, size=n).astype(np.int32) * (rng.random(n) < 0.1)
+    return f32_round(x), f32_round(params), np.diag(edges), plane.astype(np.int32), offset.astype(np.int32)
+
+
+def _fixed(impl, x, p, box, lam, flags=(True, True, True, True)):
+    out = impl._execute_fixed(x, p, box, lam, *flags)
+    # per-atom energies and du_dl: only their sums are defined
+    return [None if o is None else (o if k < 2 else o.sum(dtype=np.uint64)) for k, o in enumerate(out)]
+
+
+def _assert_same(a, b):
+    for name, u, v in zip(("du_dx", "du_dp", "du_dl", "u"), a, b):
+        if u is not None:
+            np.testing.assert_array_equal(u, v, err_msg=name)
+
+
+@pytest.mark.parametrize("n", [1, 2, 15, 16, 17, 31, 33, 65, 257, 1001])
+@pytest.mark.parametrize("rows,precision", [(8, np.float32), (16, np.float32), (32, np.float32), (16, np.float64)])
+@pytest.mark.parametrize("images", [0, 3])
+def test_all_pairs_equals_pair_list(n, rows, precision, images):
+    x, p, box, plane, offset = _case(n, 100 * n + images, images)
+    cutoff, beta = 1.2, 2.0
+    impl = P.NonbondedAllPairs(plane, offset, beta, cutoff).unbound_impl(precision)
+    if precision == np.float32:
+        impl.set_tile_rows(rows)
+    i, j = np.triu_indices(n, 1)
+    pairs = np.stack([i, j], axis=1).astype(np.int32)
+    ref = P.NonbondedPairList(pairs, np.ones((len(pairs), 2)), plane, offset, beta, cutoff).unbound_impl(precision)
+    want = _fixed(ref, x, p, box, 0.3)
+    _assert_same(_fixed(impl, x, p, box, 0.3), want)
+    # moved within the list's padding: the columns keep the order of the old distances
+    moved = f32_round(x + np.random.default_rng(n).uniform(-0.02, 0.02, size=x.shape))
+    _assert_same(_fixed(impl, moved, p, box, 0.3), _fixed(ref, moved, p, box, 0.3))
+    for flags in P.all_flag_combinations():
+        if any(flags):
+            _assert_same(_fixed(impl, moved, p, box, 0.3, flags), _fixed(ref, moved, p, box, 0.3))
+
+
+@pytest.mark.parametrize("interpolated", [False, True])
+def test_dense_group_fills_the_column_buffer(interpolated):
+    """16 + 3 row atoms with about 6,000 column atoms in reach: more than the
+    list builder sorts at once."""
+    n, nr = 6019, 19
+    rng = np.random.default_rng(5)
+    edge = 3.0
+    x = rng.uniform(0, edge, size=(n, 3))
+    x[:nr] = edge / 2 + rng.uniform(-0.1, 0.1, size=(nr, 3))
+    x = f32_round(x)
+    params = f32_round(random_params(rng, n))
+    if interpolated:
+        params = np.concatenate([params, f32_round(params * rng.uniform(0.5, 1.5, size=params.shape))])
+    plane = np.zeros(n, np.int32)
+    offset = (np.arange(n) < 5).astype(np.int32)
+    box, cutoff, beta = np.eye(3) * edge, 1.39, 2.0
+    rows = np.arange(nr, dtype=np.int32)
+    pairs = np.stack(np.meshgrid(rows, np.arange(nr, n), indexing="ij"), axis=-1).reshape(-1, 2).astype(np.int32)
+    group = P.NonbondedInteractionGroupInterpolated if interpolated else P.NonbondedInteractionGroup
+    plist = P.NonbondedPairListInterpolated if interpolated else P.NonbondedPairList
+    impl = group(rows, plane, offset, beta, cutoff).unbound_impl(np.float32)
+    ref = plist(pairs, np.ones((len(pairs), 2)), plane, offset, beta, cutoff).unbound_impl(np.float32)
+    for lam in (0.0, 0.4):
+        _assert_same(_fixed(impl, x, params, box, lam), _fixed(ref, x, params, box, lam))
+    _, tiles, _ = impl.get_nblist()
+    got = [np.sort(t) for t in tiles]
+    assert max(len(t) for t in got) > 3072
+    assert all(len(np.unique(t)) == len(t) for t in got)

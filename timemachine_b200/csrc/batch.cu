@@ -315,9 +315,11 @@ __global__ void __launch_bounds__(TB_WARPS * 32, TMNB_TB_CTAS)
         ta.n_row_blocks = r.NG;
         ta.cb_first = 0;
         ta.radius = (float)(r.cutoff + r.padding + 1e-5);
+        ta.cutoff = (float)r.cutoff;
         ta.box = r.box;
         ta.posw = r.posw;
         ta.prm = r.prm;
+        ta.lamdep = r.lamdep;
         ta.bb_ctr = r.bb_ctr;
         ta.bb_ext = r.bb_ext;
         ta.tile_cols = r.tile_cols;
@@ -396,32 +398,21 @@ __device__ __forceinline__ PairArgs pair_args(const Rep &r) {
 
 // Persistent pair kernel over every replica's work units.
 template <bool U, bool DX, bool DL, bool DP, int RG>
-__global__ void __launch_bounds__(
-    128, (DX && !U && !DL && !DP) ? (TMNB_PACKED_FORCES && RG == 16 ? TMNB_PACKED_FORCES_CTAS : 8) : 5)
+__global__ void __launch_bounds__(128, (pair_min_ctas<float, U, DX, DL, DP, false, RG>()))
     k_b_pair(const Rep *__restrict__ reps, int R, const int *__restrict__ prefix, int *counter) {
-    // forces-only evaluations of 16-row tiles take the packed sweep, as in k_pair
-    constexpr bool PACKED = TMNB_PACKED_FORCES && RG == 16 && DX && !U && !DL && !DP;
+    __shared__ WalkRows<float, DX, DP, false, RG> rows[4];
+    WalkRows<float, DX, DP, false, RG> &sm = rows[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
+    walk_clear(sm, lane);
     const int total = prefix[R];
-    for (;;) {
-        int unit = 0;
-        if (lane == 0) {
-            unit = atomicAdd(counter, 1);
-        }
-        unit = __shfl_sync(FULL_MASK, unit, 0);
-        if (unit >= total) {
-            break;
-        }
+    const int n_warps = gridDim.x * (blockDim.x / TILE);
+    for (int unit = (blockIdx.x * blockDim.x + threadIdx.x) / TILE; unit < total;
+         unit = next_unit(counter, n_warps, lane)) {
         const int q = replica_of(prefix, R, unit);
         const Rep &r = reps[q];
         const PairArgs a = pair_args(r);
         const int local = unit - prefix[q];
-        const float box_x = (float)r.box[0], box_y = (float)r.box[4], box_z = (float)r.box[8];
-        const float inv_box_x = 1 / box_x, inv_box_y = 1 / box_y, inv_box_z = 1 / box_z;
-        const float real_cutoff = (float)r.cutoff;
-        const float cutoff_squared = real_cutoff * real_cutoff;
-        const float beta = (float)r.beta;
-        const unsigned S = (unsigned)r.N;
+        const WalkBox<float> b = walk_box<float>(r.box, r.cutoff, r.beta);
         const int n_items = r.state->n_items;
         if (local >= n_items) {
             const int pair = (local - n_items) * TILE + lane;
@@ -429,33 +420,11 @@ __global__ void __launch_bounds__(
                 const int si = r.slot_of[r.pair_idxs[2 * pair + 0]];
                 const int sj = r.slot_of[r.pair_idxs[2 * pair + 1]];
                 scaled_pair<float, U, DX, DL, DP, false>(
-                    a, pair, si, sj, 0, a.acc, box_x, box_y, box_z, inv_box_x, inv_box_y, inv_box_z, cutoff_squared);
+                    a, pair, si, sj, 0, a.acc, b.x, b.y, b.z, b.inv_x, b.inv_y, b.inv_z, b.cutoff_squared);
             }
             continue;
         }
-        const int4 it = r.items[local];
-        if constexpr (PACKED) {
-            const unsigned ia = (unsigned)(it.x * RG + (lane & 7));
-            RowForces A, B;
-            for (int t = 0; t < it.z; t++) {
-                const long long tile = (long long)it.y + t;
-                const unsigned j = r.tile_cols[tile * TILE + lane];
-                tile_forces_p2<U, DX>(a, lane, S, ia, j, 0, a.acc, box_x, box_y, box_z, inv_box_x, inv_box_y, inv_box_z,
-                               cutoff_squared, beta, A, B);
-            }
-            flush_forces_p2<U, DX>(a.acc, ia, S, A, B);
-            continue;
-        }
-        const unsigned i = (unsigned)(it.x * RG + (lane & (RG - 1)));
-        unsigned long long gi_x = 0, gi_y = 0, gi_z = 0, g_qi = 0, g_sigi = 0, g_epsi = 0, du_dl = 0, energy = 0;
-        for (int t = 0; t < it.z; t++) {
-            const long long tile = (long long)it.y + t;
-            const unsigned j = r.tile_cols[tile * TILE + lane];
-            tile_pass<float, U, DX, DL, DP, false, RG>(
-                a, lane, S, i, j, 0, a.acc, box_x, box_y, box_z, inv_box_x, inv_box_y, inv_box_z, cutoff_squared, beta,
-                gi_x, gi_y, gi_z, g_qi, g_sigi, g_epsi, du_dl, energy);
-        }
-        flush_row_rg<RG, U, DX, DL, DP>(a.acc, i, i < S, gi_x, gi_y, gi_z, g_qi, g_sigi, g_epsi, du_dl, energy);
+        walk_item<float, U, DX, DL, DP, false, false, RG>(a, sm, lane, r.items[local], 0, b, a.acc);
     }
 }
 

@@ -31,27 +31,16 @@ namespace tmb {
 constexpr unsigned FULL_MASK = 0xffffffffu;
 constexpr int TILE = 32;
 
-// Forces-only FP32 evaluations of 16-row tiles use the packed two-rows-per-lane
-// sweep (sweep_forces_p2); 0 selects the one-row sweep for them too. Measured
-// on B200 (bit-identical results): MD step of the 22,840-atom box 137.9 ->
-// 132.9 us, batched MD step of 128 replicas 4.14 -> 3.93 ms. The packed
-// kernels run at 6 CTAs/SM (80 registers); 5 measured slower.
-#ifndef TMNB_PACKED_FORCES
-#define TMNB_PACKED_FORCES 1
+// CTAs per SM that the pair kernel's registers must fit: force / energy
+// outputs, with parameter derivatives, FP64.
+#ifndef TMNB_WALK_CTAS
+#define TMNB_WALK_CTAS 6
 #endif
-#ifndef TMNB_PACKED_FORCES_CTAS
-#define TMNB_PACKED_FORCES_CTAS 6
+#ifndef TMNB_WALK_CTAS_ALL
+#define TMNB_WALK_CTAS_ALL 6
 #endif
-// Energy-only FP32 evaluations of 16-row tiles (the barostat's) use the same
-// packed sweep.
-#ifndef TMNB_PACKED_ENERGY
-#define TMNB_PACKED_ENERGY 1
-#endif
-// The one-row sweep evaluates the independent x / y steps of a pair (minimum
-// image, force components) and the paired charge / epsilon derivatives in
-// the two components of packed FP32x2 operations.
-#ifndef TMNB_PACKED_SCALAR
-#define TMNB_PACKED_SCALAR 1
+#ifndef TMNB_WALK_CTAS_F64
+#define TMNB_WALK_CTAS_F64 5
 #endif
 
 // Sticky device-side state of one potential instance.
@@ -526,22 +515,6 @@ __device__ __forceinline__ void lj_first_warp(
     __syncwarp();
 }
 
-// Writes one tile's 32 column slots with the LJ atoms first (prm: staged
-// parameters, eps in .z; nullptr keeps the order).
-__device__ __forceinline__ void store_tile_lj_first(
-    unsigned *__restrict__ dst, unsigned s, unsigned S, const float4 *__restrict__ prm) {
-    const int lane = threadIdx.x & 31;
-    if (prm == nullptr) {
-        dst[lane] = s;
-        return;
-    }
-    const bool lj = s < S && prm[s].z != 0.f;
-    const unsigned m = __ballot_sync(FULL_MASK, lj);
-    const unsigned lt = (1u << lane) - 1u;
-    const int pos = lj ? __popc(m & lt) : __popc(m) + __popc(~m & lt);
-    dst[pos] = s;
-}
-
 // Bounding box of the 32-slot block rb (one warp).
 __device__ __forceinline__ void block_bounds_warp(
     int S,
@@ -614,9 +587,15 @@ static __global__ void k_block_bounds(
 // the one holding the group's first slot on (upper triangle) whose bounding
 // box is within the list radius of the group's box, each column atom at or
 // after the group's first slot is kept when any row atom lies within the list
-// radius (minimum image, 3D). Kept atoms are packed 32 to a tile, so a tile is
-// rows x 32 pairs; smaller row groups sit in smaller regions and list fewer
-// out-of-range column atoms. The tiles of row group g occupy a fixed range
+// radius (minimum image, 3D). Kept atoms are sorted (lambda-dependent atoms
+// first, then Lennard-Jones atoms, each by the number of row atoms within the
+// cutoff, most first) and packed 32 to a tile, so a tile is rows x 32 pairs and
+// its columns have about equally many pairs, which is what the pair kernel's
+// lanes wait for (of the lane steps of a 22,840-atom water box 0.80 hold a
+// pair, 0.52 with the columns in slot order). The lambda-dependent columns
+// share tiles, so fewer tiles are evaluated once per window, and most tiles
+// without Lennard-Jones columns skip that part. Smaller row groups sit in
+// smaller regions and list fewer out-of-range column atoms. The tiles of row group g occupy a fixed range
 // (tile_base) sized by the column blocks it can reach. Each group's CTA cuts
 // its tiles into work items of at most `chunk` tiles, written at a range it
 // reserves from a counter; the last CTA to finish publishes the item count.
@@ -633,9 +612,11 @@ struct TileArgs {
     int n_row_blocks; // row groups: ceil(row_end/rows)
     int cb_first;     // group: first column block (col_begin/32)
     float radius;     // list radius (cutoff + padding + margin)
+    float cutoff;     // the column order counts the row atoms within it
     const double *box;
     const float4 *posw;
-    const float4 *prm;     // staged parameters (eps in .z) to put LJ atoms first in a tile; nullptr: keep order
+    const float4 *prm;           // staged parameters (eps in .z)
+    const unsigned char *lamdep; // [S] lambda dependence of the slots' atoms
     const float4 *bb_ctr;
     const float4 *bb_ext;
     unsigned *tile_cols;   // [capacity*32] slot of each column atom (S = empty)
@@ -666,6 +647,12 @@ __host__ __device__ __forceinline__ long long tile_base(const TileArgs &a, int g
 }
 
 constexpr int TB_WARPS = 8;
+// Column atoms the CTA holds before it sorts them into tiles; a full buffer is
+// sorted and its whole tiles are written. Groups of 16 rows list about 900
+// atoms at 100 atoms per nm^3.
+constexpr int TB_COLS = 3072;
+// sort keys: lambda dependence x Lennard-Jones x 33 row counts
+constexpr int TB_KEYS = 2 * 2 * 33;
 // Tile-build CTAs per SM the compiler must fit (40 registers). The packed row
 // tests left to the compiler take 57 registers (4 CTAs/SM): measured on B200,
 // one rebuild 87.3 us with the scalar tests, 90.0 us packed at 57 registers,
@@ -674,20 +661,88 @@ constexpr int TB_WARPS = 8;
 #define TMNB_TB_CTAS 6
 #endif
 
-__device__ __forceinline__ void build_tiles_cta(const TileArgs &a, const int rb, DevState *state) {
-    __shared__ float4 row_pos[TILE];
+struct TileBuildSmem {
+    float4 row_pos[TILE];
     // the same positions as x, y, z arrays: element pair m holds rows 2m, 2m + 1
-    __shared__ __align__(8) float row_x[TILE];
-    __shared__ __align__(8) float row_y[TILE];
-    __shared__ __align__(8) float row_z[TILE];
-    __shared__ float4 row_box[2]; // the row group's box: centre, half-extent
-    __shared__ unsigned buf[TB_WARPS][2 * TILE];
-    __shared__ unsigned rem[TB_WARPS * TILE];
-    __shared__ int cand[TB_WARPS * 32]; // column blocks of the current window that pass the box test
-    __shared__ int warp_pass[TB_WARPS];
-    __shared__ int tile_count;
-    __shared__ int rem_count;
-    __shared__ int is_last;
+    // (rows past the group's last lie out of every column's reach)
+    alignas(8) float row_x[TILE];
+    alignas(8) float row_y[TILE];
+    alignas(8) float row_z[TILE];
+    float4 row_box[2]; // the row group's box: centre, half-extent
+    unsigned cols[TB_COLS];
+    unsigned char keys[TB_COLS];
+    unsigned rem_cols[TILE];
+    unsigned char rem_keys[TILE];
+    int bins[TB_KEYS]; // columns of each key, then the next position of each key
+    int n_cols;
+    int cand[TB_WARPS * 32]; // column blocks of the current window that pass the box test
+    int warp_pass[TB_WARPS];
+    int is_last;
+};
+
+// Sorts the CTA's n collected columns by key and writes them as tiles from
+// first_tile on: all of them (the last tile padded with S) when `last`,
+// else the whole tiles, keeping the rest collected. Returns the tiles written.
+__device__ __forceinline__ int tb_emit(TileBuildSmem &sm, const TileArgs &a, int n, long long first_tile, bool last) {
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x < TILE) {
+        constexpr int PER = (TB_KEYS + TILE - 1) / TILE;
+        int c[PER], sum = 0;
+        for (int k = 0; k < PER; k++) {
+            const int b = lane * PER + k;
+            c[k] = b < TB_KEYS ? sm.bins[b] : 0;
+            sum += c[k];
+        }
+        int incl = sum;
+        for (int o = 1; o < TILE; o <<= 1) {
+            const int v = __shfl_up_sync(FULL_MASK, incl, o);
+            incl += lane >= o ? v : 0;
+        }
+        int at = incl - sum;
+        for (int k = 0; k < PER; k++) {
+            const int b = lane * PER + k;
+            if (b < TB_KEYS) {
+                sm.bins[b] = at;
+            }
+            at += c[k];
+        }
+    }
+    __syncthreads();
+    const int n_out = last ? (n + TILE - 1) / TILE * TILE : n / TILE * TILE;
+    unsigned *dst = a.tile_cols + first_tile * TILE;
+    for (int k = threadIdx.x; k < n; k += TB_WARPS * 32) {
+        const int pos = atomicAdd(&sm.bins[sm.keys[k]], 1);
+        if (pos < n_out) {
+            dst[pos] = sm.cols[k];
+        } else {
+            sm.rem_cols[pos - n_out] = sm.cols[k];
+            sm.rem_keys[pos - n_out] = sm.keys[k];
+        }
+    }
+    if (n + (int)threadIdx.x < n_out) {
+        dst[n + threadIdx.x] = (unsigned)a.S;
+    }
+    __syncthreads();
+    if (!last) {
+        for (int k = threadIdx.x; k < TB_KEYS; k += TB_WARPS * 32) {
+            sm.bins[k] = 0;
+        }
+        __syncthreads();
+        if ((int)threadIdx.x < n - n_out) {
+            sm.cols[threadIdx.x] = sm.rem_cols[threadIdx.x];
+            sm.keys[threadIdx.x] = sm.rem_keys[threadIdx.x];
+            atomicAdd(&sm.bins[sm.rem_keys[threadIdx.x]], 1);
+        }
+        if (threadIdx.x == 0) {
+            sm.n_cols = n - n_out;
+        }
+        __syncthreads();
+    }
+    return n_out / TILE;
+}
+
+__device__ __forceinline__ void build_tiles_cta(const TileArgs &a, const int rb, DevState *state) {
+    __shared__ TileBuildSmem sm;
 
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
@@ -695,6 +750,7 @@ __device__ __forceinline__ void build_tiles_cta(const TileArgs &a, const int rb,
     const float Lx = (float)a.box[0], Ly = (float)a.box[4], Lz = (float)a.box[8];
     const float iLx = 1.0f / Lx, iLy = 1.0f / Ly, iLz = 1.0f / Lz;
     const float r2 = a.radius * a.radius;
+    const float rc2 = a.cutoff * a.cutoff;
     const float r2_box = (a.radius + 1e-4f) * (a.radius + 1e-4f);
     const int rows = a.rows;
     const int row_first = rb * rows;
@@ -720,15 +776,15 @@ __device__ __forceinline__ void build_tiles_cta(const TileArgs &a, const int rb,
             mxz = fmaxf(mxz, __shfl_xor_sync(FULL_MASK, mxz, o));
         }
         if (lane == 0) {
-            row_box[0] = make_float4(rx + 0.5f * (mnx + mxx), ry + 0.5f * (mny + mxy), rz + 0.5f * (mnz + mxz), 0.f);
-            row_box[1] = make_float4(
+            sm.row_box[0] = make_float4(rx + 0.5f * (mnx + mxx), ry + 0.5f * (mny + mxy), rz + 0.5f * (mnz + mxz), 0.f);
+            sm.row_box[1] = make_float4(
                 0.5f * (mxx - mnx) * 1.000001f + 1e-6f, 0.5f * (mxy - mny) * 1.000001f + 1e-6f,
                 0.5f * (mxz - mnz) * 1.000001f + 1e-6f, 0.f);
         }
     }
     __syncthreads();
-    const float4 rc = row_box[0];
-    const float4 re = row_box[1];
+    const float4 rc = sm.row_box[0];
+    const float4 re = sm.row_box[1];
 
     // Row atoms are imaged next to the row block's centre. When every box
     // edge satisfies L/2 - extent >= radius, a column atom imaged next to the
@@ -742,28 +798,28 @@ __device__ __forceinline__ void build_tiles_cta(const TileArgs &a, const int rb,
         p.x = rc.x + wrap_delta(p.x - rc.x, Lx, iLx);
         p.y = rc.y + wrap_delta(p.y - rc.y, Ly, iLy);
         p.z = rc.z + wrap_delta(p.z - rc.z, Lz, iLz);
-        row_pos[threadIdx.x] = p;
-        row_x[threadIdx.x] = p.x;
-        row_y[threadIdx.x] = p.y;
-        row_z[threadIdx.x] = p.z;
+        sm.row_pos[threadIdx.x] = p;
+        sm.row_x[threadIdx.x] = (int)threadIdx.x < row_n ? p.x : 1e18f;
+        sm.row_y[threadIdx.x] = p.y;
+        sm.row_z[threadIdx.x] = p.z;
+    }
+    for (int k = threadIdx.x; k < TB_KEYS; k += TB_WARPS * 32) {
+        sm.bins[k] = 0;
     }
     if (threadIdx.x == 0) {
-        tile_count = 0;
-        rem_count = 0;
+        sm.n_cols = 0;
     }
     __syncthreads();
     const int col_lo = a.group ? a.col_begin : row_first; // first column slot of the group's pairs
     const long long base_tile = tile_base(a, rb);
     const unsigned lane_lt = (1u << lane) - 1;
 
-    int count = 0; // atoms in this warp's buffer
+    int tiles = 0;  // tiles written so far (uniform over the CTA)
+    int n_have = 0; // columns collected (uniform over the CTA)
     // Column blocks in windows of one block per thread: the box test of the
     // window compacts the passing blocks in index order, then each warp takes
-    // an equal contiguous share of them. Passing blocks cluster at nearby
-    // indices, so a fixed split of the window by index would leave most warps
-    // idle; contiguous shares keep each warp's tiles spatially compact (the
-    // slot order is a space-filling curve), which the pair kernel's
-    // divergence depends on.
+    // an equal share of them. Passing blocks cluster at nearby indices, so a
+    // fixed split of the window by index would leave most warps idle.
     for (int wbase = a.group ? a.cb_first : row_first / TILE; wbase < a.RB; wbase += TB_WARPS * 32) {
         const int cb = wbase + (int)threadIdx.x;
         bool pass = false;
@@ -777,115 +833,100 @@ __device__ __forceinline__ void build_tiles_cta(const TileArgs &a, const int rb,
         }
         const unsigned m = __ballot_sync(FULL_MASK, pass);
         if (lane == 0) {
-            warp_pass[warp] = __popc(m);
+            sm.warp_pass[warp] = __popc(m);
         }
         __syncthreads();
         int base = 0, nc = 0;
         for (int w = 0; w < TB_WARPS; w++) {
-            const int c = warp_pass[w];
+            const int c = sm.warp_pass[w];
             base += w < warp ? c : 0;
             nc += c;
         }
         if (pass) {
-            cand[base + __popc(m & lane_lt)] = cb;
+            sm.cand[base + __popc(m & lane_lt)] = cb;
         }
         __syncthreads();
-        const int k_end = ((warp + 1) * nc) / TB_WARPS;
-        for (int k = (warp * nc) / TB_WARPS; k < k_end; k++) {
-            const int cb_sel = cand[k];
-            const int s = cb_sel * TILE + lane;
-            const bool valid = s < S;
-            const float4 pj = valid ? a.posw[s] : make_float4(0.f, 0.f, 0.f, 0.f);
-            // an atom farther than the radius from the row block's box is
-            // farther than the radius from every row atom (widened test,
-            // conservative under rounding): skip its per-row test
-            const float wx = wrap_delta(pj.x - rc.x, Lx, iLx);
-            const float wy = wrap_delta(pj.y - rc.y, Ly, iLy);
-            const float wz = wrap_delta(pj.z - rc.z, Lz, iLz);
-            const float bx = fmaxf(0.f, fabsf(wx) - re.x);
-            const float by = fmaxf(0.f, fabsf(wy) - re.y);
-            const float bz = fmaxf(0.f, fabsf(wz) - re.z);
-            const bool need = valid && s >= col_lo && bx * bx + by * by + bz * bz < r2_box;
-            bool hit = false;
-            if (__any_sync(FULL_MASK, need)) {
+        for (int k0 = 0; k0 < nc;) {
+            if (TB_COLS - n_have < TB_WARPS * TILE) {
+                tiles += tb_emit(sm, a, n_have, base_tile + tiles, false);
+                n_have = n_have % TILE;
+            }
+            const int take = min(nc - k0, (TB_COLS - n_have) / TILE); // blocks whose atoms all fit
+            const int k_end = k0 + ((warp + 1) * take) / TB_WARPS;
+            for (int k = k0 + (warp * take) / TB_WARPS; k < k_end; k++) {
+                const int s = sm.cand[k] * TILE + lane;
+                const bool valid = s < S;
+                const float4 pj = valid ? a.posw[s] : make_float4(0.f, 0.f, 0.f, 0.f);
+                // an atom farther than the radius from the row block's box is
+                // farther than the radius from every row atom (widened test,
+                // conservative under rounding): skip its per-row test
+                const float wx = wrap_delta(pj.x - rc.x, Lx, iLx);
+                const float wy = wrap_delta(pj.y - rc.y, Ly, iLy);
+                const float wz = wrap_delta(pj.z - rc.z, Lz, iLz);
+                const float bx = fmaxf(0.f, fabsf(wx) - re.x);
+                const float by = fmaxf(0.f, fabsf(wy) - re.y);
+                const float bz = fmaxf(0.f, fabsf(wz) - re.z);
+                const bool need = valid && s >= col_lo && bx * bx + by * by + bz * bz < r2_box;
+                if (!__any_sync(FULL_MASK, need)) {
+                    continue;
+                }
+                float d2_min = 3.0e38f;
+                int near = 0; // row atoms within the cutoff
                 if (shifted) {
-                    // two rows per packed FP32x2 test (rows past row_n sit at
-                    // the centre and are masked)
+                    // two rows per packed FP32x2 test
                     const float2 qx = f2(rc.x + wx), qy = f2(rc.y + wy), qz = f2(rc.z + wz);
-                    const float2 *rx2 = reinterpret_cast<const float2 *>(row_x);
-                    const float2 *ry2 = reinterpret_cast<const float2 *>(row_y);
-                    const float2 *rz2 = reinterpret_cast<const float2 *>(row_z);
-                    for (int r0 = 0; r0 < row_n; r0 += 8) {
+                    const float2 *rx2 = reinterpret_cast<const float2 *>(sm.row_x);
+                    const float2 *ry2 = reinterpret_cast<const float2 *>(sm.row_y);
+                    const float2 *rz2 = reinterpret_cast<const float2 *>(sm.row_z);
+                    for (int r0 = 0; r0 < rows; r0 += 8) {
 #pragma unroll
                         for (int r = r0; r < r0 + 8; r += 2) {
                             const float2 dx = fsub2(rx2[r >> 1], qx);
                             const float2 dy = fsub2(ry2[r >> 1], qy);
                             const float2 dz = fsub2(rz2[r >> 1], qz);
                             const float2 d2 = ffma2(dz, dz, ffma2(dy, dy, fmul2(dx, dx)));
-                            hit |= ((r < row_n) && (d2.x < r2)) || ((r + 1 < row_n) && (d2.y < r2));
-                        }
-                        if (__all_sync(FULL_MASK, hit || !need)) {
-                            break;
+                            d2_min = fminf(d2_min, fminf(d2.x, d2.y));
+                            near += d2.x < rc2 ? 1 : 0;
+                            near += d2.y < rc2 ? 1 : 0;
                         }
                     }
                 } else {
-                    // rows in groups of 8 (independent tests, then one vote)
-                    for (int r0 = 0; r0 < row_n; r0 += 8) {
-#pragma unroll
-                        for (int r = r0; r < r0 + 8; r++) {
-                            const float4 pi = row_pos[r];
-                            const float dx = wrap_delta(pi.x - pj.x, Lx, iLx);
-                            const float dy = wrap_delta(pi.y - pj.y, Ly, iLy);
-                            const float dz = wrap_delta(pi.z - pj.z, Lz, iLz);
-                            hit |= (r < row_n) && (dx * dx + dy * dy + dz * dz < r2);
-                        }
-                        if (__all_sync(FULL_MASK, hit || !need)) {
-                            break;
-                        }
+                    for (int r = 0; r < row_n; r++) {
+                        const float4 pi = sm.row_pos[r];
+                        const float dx = wrap_delta(pi.x - pj.x, Lx, iLx);
+                        const float dy = wrap_delta(pi.y - pj.y, Ly, iLy);
+                        const float dz = wrap_delta(pi.z - pj.z, Lz, iLz);
+                        const float d2 = dx * dx + dy * dy + dz * dz;
+                        d2_min = fminf(d2_min, d2);
+                        near += d2 < rc2 ? 1 : 0;
                     }
                 }
-            }
-            hit = hit && need;
-            const unsigned hmask = __ballot_sync(FULL_MASK, hit);
-            if (hit) {
-                buf[warp][count + __popc(hmask & lane_lt)] = (unsigned)s;
-            }
-            count += __popc(hmask);
-            __syncwarp();
-            if (count >= TILE) {
-                int t = 0;
-                if (lane == 0) {
-                    t = atomicAdd(&tile_count, 1);
+                const bool hit = need && d2_min < r2;
+                const unsigned hmask = __ballot_sync(FULL_MASK, hit);
+                if (hmask == 0) {
+                    continue;
                 }
-                t = __shfl_sync(FULL_MASK, t, 0);
-                store_tile_lj_first(a.tile_cols + (base_tile + t) * TILE, buf[warp][lane], (unsigned)S, a.prm);
-                __syncwarp();
-                buf[warp][lane] = buf[warp][TILE + lane];
-                __syncwarp();
-                count -= TILE;
+                int at = 0;
+                if (lane == 0) {
+                    at = atomicAdd(&sm.n_cols, __popc(hmask));
+                }
+                at = __shfl_sync(FULL_MASK, at, 0) + __popc(hmask & lane_lt);
+                if (hit) {
+                    const int key = (a.lamdep[s] ? 0 : 66) + (a.prm[s].z != 0.f ? 0 : 33) + 32 - near;
+                    sm.cols[at] = (unsigned)s;
+                    sm.keys[at] = (unsigned char)key;
+                    atomicAdd(&sm.bins[key], 1);
+                }
             }
+            k0 += take;
+            __syncthreads();
+            n_have = sm.n_cols;
+            __syncthreads(); // read by all before the next columns are added
         }
-        __syncthreads(); // cand / warp_pass are rewritten by the next window
     }
-    // merge the partial buffers of the warps
-    int off = 0;
-    if (lane == 0) {
-        off = atomicAdd(&rem_count, count);
-    }
-    off = __shfl_sync(FULL_MASK, off, 0);
-    if (lane < count) {
-        rem[off + lane] = buf[warp][lane];
-    }
-    __syncthreads();
+    tiles += tb_emit(sm, a, n_have, base_tile + tiles, true);
     if (warp == 0) {
-        const int n = rem_count;
-        for (int b = 0; b < n; b += TILE) {
-            const int t = tile_count + b / TILE;
-            store_tile_lj_first(a.tile_cols + (base_tile + t) * TILE, b + lane < n ? rem[b + lane] : (unsigned)S,
-                                (unsigned)S, a.prm);
-        }
-        __syncwarp();
-        const int total = tile_count + (n + TILE - 1) / TILE;
+        const int total = tiles;
         // the group's work items, at a range reserved from the list's
         // counter (items are in any order: the pair kernel schedules them
         // dynamically and its sums do not depend on the order)
@@ -908,10 +949,10 @@ __device__ __forceinline__ void build_tiles_cta(const TileArgs &a, const int rb,
     __syncthreads();
     if (threadIdx.x == 0) {
         const unsigned prev = atomicAdd(&state->done_ctas, 1u);
-        is_last = (prev == (unsigned)a.n_row_blocks - 1);
+        sm.is_last = (prev == (unsigned)a.n_row_blocks - 1);
     }
     __syncthreads();
-    if (!is_last) {
+    if (!sm.is_last) {
         return;
     }
     if (threadIdx.x == 0) {
@@ -1017,262 +1058,463 @@ template <> struct Staged<double> {
     }
 };
 
-// The arithmetic of one in-range pair (row atom i, column atom j) from its
-// minimum-image deltas and 4D d2: adds the row's and the column's fixed-point
-// contributions. Every sweep calls this one function, so a pair rounds the
-// same whichever schedule evaluates it. Per-pair arithmetic and validity follow
-// timemachine/cpp/src/kernels/k_nonbonded.cuh:424-546; the column
-// contribution of du_dx is the exact negation of the row contribution
-// (llrint is odd under round-half-even), so it is converted once.
-template <typename Real, bool U, bool DX, bool DL, bool DP, bool INTERP, bool ALCH>
-__device__ __forceinline__ void pair_terms(
-    const Real delta_x,
-    const Real delta_y,
-    const Real delta_z,
-    const Real delta_w,
-    const Real d2,
-    const Real qi,
-    const Real sig_i,
-    const Real eps_i,
-    const Real dw_dl_i,
-    const Real dq_dl_i,
-    const Real dsig_dl_i,
-    const Real deps_dl_i,
-    const Real qj,
-    const Real sig_j,
-    const Real eps_j,
-    const Real dw_dl_j,
-    const Real dq_dl_j,
-    const Real dsig_dl_j,
-    const Real deps_dl_j,
-    const Real beta,
-    unsigned long long &gi_x,
-    unsigned long long &gi_y,
-    unsigned long long &gi_z,
-    unsigned long long &g_qi,
-    unsigned long long &g_sigi,
-    unsigned long long &g_epsi,
-    unsigned long long &du_dl,
-    unsigned long long &energy,
-    unsigned long long &gj_x,
-    unsigned long long &gj_y,
-    unsigned long long &gj_z,
-    unsigned long long &g_qj,
-    unsigned long long &g_sigj,
-    unsigned long long &g_epsj) {
-    Real u;
-    Real prefactor;
-    Real erfc_bd;
-    Real d;
-    Real inv_d;
-    Real inv_d2;
-    Real qij_inv;
-    Real factor;
-    electrostatics<Real, U>((Real)1, qi, qj, d2, beta, d, inv_d, inv_d2, erfc_bd, prefactor, u, qij_inv, factor);
-    Real real_du_dl = 0;
-    if (eps_i != 0 && eps_j != 0) {
-        Real sig_grad;
-        Real eps_grad;
-        lennard_jones<Real, U>(
-            (Real)1, eps_i, eps_j, sig_i, sig_j, inv_d, inv_d2, qij_inv, factor, erfc_bd, u, prefactor, sig_grad,
-            eps_grad);
-        if (DP) {
-            const unsigned long long gs = to_fixed(sig_grad, FX_EXPONENT_SIG);
-            g_sigi += gs;
-            g_sigj += gs;
-            if constexpr (TMNB_PACKED_SCALAR && sizeof(Real) == 4) {
-                const float2 ge = fmul2(fmul2(f2(eps_grad), make_float2(eps_j, eps_i)),
-                                        f2(static_cast<float>(FX_EXPONENT_EPS)));
-                g_epsi += fixed_round(ge.x);
-                g_epsj += fixed_round(ge.y);
-            } else {
-                g_epsi += to_fixed(fmul(eps_grad, eps_j), FX_EXPONENT_EPS);
-                g_epsj += to_fixed(fmul(eps_grad, eps_i), FX_EXPONENT_EPS);
+// ---------------------------------------------------------------------------
+// Tile walk: the pairs of a tile (RG rows x 32 columns) that lie within the
+// cutoff, and only those.
+//
+// What bounds it: instruction issue, then the shared-memory pipe (ncu, forces
+// at 22,840 atoms: 71 % of issue slots, 28 of 32 lanes per instruction, shared
+// wavefronts half of the pipe's cycles; DRAM idle). The sweep of every row x
+// column that this replaced issued 69.8 M warp instructions there, the walk
+// 49.6 M. Kernel times on B200, before -> after, bit-identical: all outputs of
+// 12 windows at 22,840 atoms 157 -> 109 us (FP64 363 -> 239), forces of an MD
+// step 80.5 -> 68, all outputs at 98,000 atoms 480 -> 322; batch of 24 replicas
+// 1,568 -> 1,171 (all), 1,017 -> 795 (forces). 7 or 8 CTAs/SM instead of 6
+// change nothing; loading the next tile's columns ahead costs 2 to 6 %.
+//
+// Lane l owns column l of the tile: its atom and its sums stay in registers.
+// The tile's rows are staged in shared memory once per work item. A tile takes
+// two passes: every lane marks the rows within the cutoff of its column (a bit
+// mask, distances only, two rows per packed FP32x2 operation), then walks its
+// own marked rows, one per step, all lanes with the pair arithmetic at once.
+// The list builder puts columns with about as many rows in range next to each
+// other, so the lanes of a tile have walks of about the same length (0.80 of
+// the lane steps hold a pair; 0.42 of the slots of the tiles do, which is what
+// a sweep over all rows x columns spends the pair arithmetic on).
+//
+// A row's sums are met by several lanes in a step and live in shared memory as
+// two 32-bit limbs (bits 0-23 and 24-55 of the fixed-point value): 32-bit
+// shared-memory additions are native, 64-bit ones are compare-and-swap loops.
+// 64 additions of values below 2^49 fit the limbs exactly; larger values (and
+// NaN) go to the row's global accumulator as a whole. Lane l starts its walk at
+// row l mod RG and each RG-lane group has its own copy of the sums, so the
+// lanes of a step mostly meet different words.
+// ---------------------------------------------------------------------------
+template <typename Real> struct alignas(2 * sizeof(Real)) Vec2 {
+    Real a, b;
+};
+
+// The rows of one work item, one instance per warp.
+template <typename Real, bool DX, bool DP, bool INTERP, int RG> struct alignas(16) WalkRows {
+    static constexpr int FIELDS = (DX ? 3 : 0) + (DP ? 3 : 0);
+    // tiles between two flushes of the row sums: at most 64 additions to a word
+    static constexpr int FLUSH_TILES = 64 / RG;
+    // coordinates row by row for the distance pass, and as pairs for the walk
+    Real x[RG], y[RG], z[RG];
+    Vec2<Real> xy[RG], zq[RG], se[RG], wd[RG]; // (x, y), (z, q), (sig, eps), (w, dw/dlambda)
+    Vec2<Real> dqs[INTERP ? RG : 1];           // (dq/dlambda, dsig/dlambda)
+    Real de[INTERP ? RG : 1];                  // deps/dlambda
+    Real lo[3], hi[3];                         // smallest and largest row coordinates
+    unsigned acc[FIELDS > 0 ? 2 * FIELDS : 1][TILE]; // limbs of the row sums: [field low, high][copy * RG + row]
+};
+
+// Sums of the lane's column.
+struct ColSums {
+    unsigned long long x = 0, y = 0, z = 0, q = 0, sig = 0, eps = 0, u = 0, dl = 0;
+};
+
+// What a tile needs besides its atoms, uniform over the launch.
+template <typename Real> struct WalkBox {
+    Real x, y, z;          // box edges
+    Real inv_x, inv_y, inv_z;
+    Real cutoff_squared, beta;
+};
+
+template <typename Real> __device__ __forceinline__ WalkBox<Real> walk_box(const double *box, double cutoff, double beta) {
+    WalkBox<Real> b;
+    b.x = box[0];
+    b.y = box[4];
+    b.z = box[8];
+    b.inv_x = 1 / b.x;
+    b.inv_y = 1 / b.y;
+    b.inv_z = 1 / b.z;
+    const Real c = static_cast<Real>(cutoff);
+    b.cutoff_squared = c * c;
+    b.beta = static_cast<Real>(beta);
+    return b;
+}
+
+// A fixed-point value that the limbs hold.
+template <typename Real> __device__ __forceinline__ bool fits_limbs(Real y) { return fabs(y) < static_cast<Real>(0x1p49); }
+
+__device__ __forceinline__ void limbs_add(unsigned (*acc)[TILE], int field, int word, unsigned long long v) {
+    atomicAdd(&acc[2 * field][word], static_cast<unsigned>(v) & 0xffffffu);
+    atomicAdd(&acc[2 * field + 1][word], static_cast<unsigned>(v >> 24));
+}
+
+template <typename Real, bool DX, bool DP, bool INTERP, int RG>
+__device__ __forceinline__ void walk_clear(WalkRows<Real, DX, DP, INTERP, RG> &sm, int lane) {
+    for (int f = 0; f < 2 * sm.FIELDS; f++) {
+        sm.acc[f][lane] = 0;
+    }
+    __syncwarp();
+}
+
+// Stages the rows row_first .. row_first + RG - 1 of one window (slots from
+// row_end on: NaN coordinates, which pass no cutoff test). Returns whether any
+// row's terms depend on lambda.
+template <typename Real, bool DX, bool DP, bool INTERP, int RG>
+__device__ __forceinline__ bool walk_load_rows(
+    const PairArgs &a, WalkRows<Real, DX, DP, INTERP, RG> &sm, const int lane, const unsigned row_first, const int window) {
+    using St = Staged<Real>;
+    using V = typename St::V;
+    const size_t wo = (size_t)window * a.S;
+    const int r = lane & (RG - 1);
+    const unsigned i = row_first + r;
+    const bool ok = i < (unsigned)a.row_end;
+    const Real nan = static_cast<Real>(__int_as_float(0x7fffffff));
+    const V pw = ok ? St::posw(a)[wo + i] : St::make(nan, nan, nan, 0);
+    const V pr = ok ? St::prm(a)[wo + i] : St::make(0, 0, 0, 0);
+    V dp = St::make(0, 0, 0, 0);
+    if (INTERP && ok) {
+        dp = St::dprm(a)[wo + i];
+    }
+    // fmin / fmax pass over the NaN rows
+    Real lx = pw.x, ly = pw.y, lz = pw.z, hx = pw.x, hy = pw.y, hz = pw.z;
+#pragma unroll
+    for (int o = RG / 2; o > 0; o >>= 1) {
+        lx = fmin(lx, __shfl_xor_sync(FULL_MASK, lx, o));
+        ly = fmin(ly, __shfl_xor_sync(FULL_MASK, ly, o));
+        lz = fmin(lz, __shfl_xor_sync(FULL_MASK, lz, o));
+        hx = fmax(hx, __shfl_xor_sync(FULL_MASK, hx, o));
+        hy = fmax(hy, __shfl_xor_sync(FULL_MASK, hy, o));
+        hz = fmax(hz, __shfl_xor_sync(FULL_MASK, hz, o));
+    }
+    __syncwarp(); // the previous item's walks are done with the rows
+    if (lane < RG) {
+        sm.x[r] = pw.x;
+        sm.y[r] = pw.y;
+        sm.z[r] = pw.z;
+        sm.xy[r] = {pw.x, pw.y};
+        sm.zq[r] = {pw.z, pr.x};
+        sm.se[r] = {pr.y, pr.z};
+        sm.wd[r] = {pw.w, pr.w};
+        if (INTERP) {
+            sm.dqs[r] = {dp.x, dp.y};
+            sm.de[r] = dp.z;
+        }
+    }
+    if (lane == 0) {
+        sm.lo[0] = lx;
+        sm.lo[1] = ly;
+        sm.lo[2] = lz;
+        sm.hi[0] = hx;
+        sm.hi[1] = hy;
+        sm.hi[2] = hz;
+    }
+    __syncwarp();
+    return __any_sync(FULL_MASK, pw.w != 0 || (INTERP && (dp.x != 0 || dp.y != 0 || dp.z != 0)));
+}
+
+// Adds the rows' sums to the accumulators of the row slots and clears them.
+template <typename Real, bool DX, bool DP, bool INTERP, int RG>
+__device__ __forceinline__ void walk_flush_rows(
+    WalkRows<Real, DX, DP, INTERP, RG> &sm, const int lane, const Accum &out, const unsigned row_first, const int row_end) {
+    __syncwarp();
+    const unsigned i = row_first + lane;
+    const bool writes = lane < RG && i < (unsigned)row_end;
+#pragma unroll
+    for (int f = 0; f < sm.FIELDS; f++) {
+        unsigned long long v = (unsigned long long)sm.acc[2 * f][lane] +
+                               ((unsigned long long)(long long)(int)sm.acc[2 * f + 1][lane] << 24);
+        sm.acc[2 * f][lane] = 0;
+        sm.acc[2 * f + 1][lane] = 0;
+#pragma unroll
+        for (int o = RG; o < TILE; o <<= 1) {
+            v += __shfl_xor_sync(FULL_MASK, v, o);
+        }
+        if (writes && v != 0) {
+            const int k = DX ? f : f + 3;
+            unsigned long long *to =
+                k == 0 ? out.x : k == 1 ? out.y : k == 2 ? out.z : k == 3 ? out.q : k == 4 ? out.sig : out.eps;
+            red_add(to + i, v);
+        }
+    }
+    __syncwarp();
+}
+
+// Minimum-image displacement of a coordinate pair: the general form, or the
+// image count of the column given as its shift (-box * count).
+template <bool WRAP, typename V2>
+__device__ __forceinline__ V2 walk_delta2(V2 ci, V2 cj, V2 shift, V2 neg_box, V2 inv_box) {
+    if (WRAP) {
+        return min_image2(fsub2(ci, cj), neg_box, inv_box);
+    }
+    return fadd2(fsub2(ci, cj), shift);
+}
+template <bool WRAP, typename Real>
+__device__ __forceinline__ Real walk_delta(Real ci, Real cj, Real shift, Real box, Real inv_box) {
+    if (WRAP) {
+        return min_image(fsub(ci, cj), box, inv_box);
+    }
+    return fadd(fsub(ci, cj), shift);
+}
+
+// One tile, columns j (one per lane; >= S: none), window `window`. Per-pair
+// arithmetic and validity follow
+// timemachine/cpp/src/kernels/k_nonbonded.cuh:424-546; the column's force is
+// the exact negation of the row's (llrint is odd under round-half-even), so it
+// is converted once. The energy and du_dl of a pair go to its column.
+template <typename Real, bool U, bool DX, bool DL, bool DP, bool INTERP, bool ALCH, bool WRAP, int RG>
+__device__ __forceinline__ void walk_pairs(
+    WalkRows<Real, DX, DP, INTERP, RG> &sm,
+    const int lane,
+    const unsigned row_first,
+    const unsigned valid_rows, // rows that pair with the lane's column at all
+    const typename Staged<Real>::V pwj,
+    const typename Staged<Real>::V prj,
+    const typename Staged<Real>::V dpj,
+    const Real shift_x,
+    const Real shift_y,
+    const Real shift_z,
+    const WalkBox<Real> &b,
+    const Accum &out,
+    ColSums &g) {
+    using V2 = decltype(f2(Real(0)));
+    // 1. rows within the cutoff of the lane's column
+    unsigned mask = 0;
+    {
+        const V2 cx = f2(pwj.x), cy = f2(pwj.y), cz = f2(pwj.z);
+        const V2 sx = f2(shift_x), sy = f2(shift_y), sz = f2(shift_z);
+#pragma unroll
+        for (int r = 0; r < RG; r += 2) {
+            const Vec2<Real> xr = *reinterpret_cast<const Vec2<Real> *>(&sm.x[r]);
+            const Vec2<Real> yr = *reinterpret_cast<const Vec2<Real> *>(&sm.y[r]);
+            const Vec2<Real> zr = *reinterpret_cast<const Vec2<Real> *>(&sm.z[r]);
+            const V2 dx = walk_delta2<WRAP>(make2(xr.a, xr.b), cx, sx, f2(-b.x), f2(b.inv_x));
+            const V2 dy = walk_delta2<WRAP>(make2(yr.a, yr.b), cy, sy, f2(-b.y), f2(b.inv_y));
+            const V2 dz = walk_delta2<WRAP>(make2(zr.a, zr.b), cz, sz, f2(-b.z), f2(b.inv_z));
+            V2 d2 = dist2(dx, dy, dz);
+            if (ALCH) {
+                const V2 dw = fsub2(make2(sm.wd[r].a, sm.wd[r + 1].a), f2(pwj.w));
+                d2 = madd2(dw, dw, d2, TMNB_DAG_D4);
+            }
+            if (d2.x < b.cutoff_squared) {
+                mask |= 1u << r;
+            }
+            if (d2.y < b.cutoff_squared) {
+                mask |= 2u << r;
             }
         }
-        if (DL && ALCH && INTERP) {
-            real_du_dl = ffma(sig_grad, fadd(dsig_dl_i, dsig_dl_j), real_du_dl);
-            real_du_dl = ffma(eps_grad, sum_of_products_rn(eps_j, deps_dl_i, eps_i, deps_dl_j), real_du_dl);
-        }
+        mask &= valid_rows;
     }
-    if (DX) {
-        // The column's term llrint(-y) equals -llrint(y) (round-half-even is
-        // odd) except where the conversion saturates (|y| >= 2^63) or y is NaN;
-        // those lanes add the difference afterwards.
-        const Real ex = static_cast<Real>(FX_EXPONENT);
-        Real yx, yy;
-        if constexpr (TMNB_PACKED_SCALAR && sizeof(Real) == 4) {
-            const float2 yxy = fmul2(fmul2(f2(prefactor), make_float2(delta_x, delta_y)), f2(ex));
-            yx = yxy.x;
-            yy = yxy.y;
-        } else {
-            yx = fmul(fmul(prefactor, delta_x), ex);
-            yy = fmul(fmul(prefactor, delta_y), ex);
+    // 2. the lane's rows, from row l mod RG on
+    const int rot = lane & (RG - 1);
+    const int copy = lane & ~(RG - 1);
+    unsigned m = RG == TILE ? __funnelshift_r(mask, mask, rot)
+                            : ((mask | (mask << (RG & 31))) >> rot) & (unsigned)((1ull << RG) - 1);
+    for (unsigned n = __reduce_max_sync(FULL_MASK, (unsigned)__popc(m)); n > 0; n--) {
+        if (m == 0) {
+            continue;
         }
-        const Real yz = fmul(fmul(prefactor, delta_z), ex);
-        const unsigned long long fx = fixed_round(yx);
-        const unsigned long long fy = fixed_round(yy);
-        const unsigned long long fz = fixed_round(yz);
-        gi_x += fx;
-        gi_y += fy;
-        gi_z += fz;
-        gj_x -= fx;
-        gj_y -= fy;
-        gj_z -= fz;
-        if (!fixed_in_range(yx) || !fixed_in_range(yy) || !fixed_in_range(yz)) {
-            gj_x += fixed_round(-yx) + fx;
-            gj_y += fixed_round(-yy) + fy;
-            gj_z += fixed_round(-yz) + fz;
+        const int r = (__ffs(m) - 1 + rot) & (RG - 1);
+        m &= m - 1;
+        const Vec2<Real> xy = sm.xy[r];
+        const Vec2<Real> zq = sm.zq[r];
+        const V2 dxy = walk_delta2<WRAP>(
+            make2(xy.a, xy.b), make2(pwj.x, pwj.y), make2(shift_x, shift_y), make2(-b.x, -b.y), make2(b.inv_x, b.inv_y));
+        const Real delta_x = dxy.x, delta_y = dxy.y;
+        const Real delta_z = walk_delta<WRAP>(zq.a, pwj.z, shift_z, b.z, b.inv_z);
+        Real d2 = dist2(delta_x, delta_y, delta_z);
+        Real delta_w = 0, dw_dl_i = 0;
+        if (ALCH) {
+            const Vec2<Real> wd = sm.wd[r];
+            delta_w = fsub(wd.a, pwj.w);
+            dw_dl_i = wd.b;
+            d2 = add_w2(d2, delta_w);
         }
-    }
-    if (DP) {
-        if constexpr (TMNB_PACKED_SCALAR && sizeof(Real) == 4) {
-            const float2 gq = fmul2(fmul2(fmul2(make_float2(qj, qi), f2(inv_d)), f2(erfc_bd)),
-                                    f2(static_cast<float>(FX_EXPONENT)));
-            g_qi += fixed_round(gq.x);
-            g_qj += fixed_round(gq.y);
-        } else {
-            g_qi += to_fixed(fmul(fmul(qj, inv_d), erfc_bd), FX_EXPONENT);
-            g_qj += to_fixed(fmul(fmul(qi, inv_d), erfc_bd), FX_EXPONENT);
+        const Real qi = zq.b, qj = prj.x;
+        Real u, prefactor, erfc_bd, d, inv_d, inv_d2, qij_inv, factor;
+        electrostatics<Real, U>((Real)1, qi, qj, d2, b.beta, d, inv_d, inv_d2, erfc_bd, prefactor, u, qij_inv, factor);
+        Real real_du_dl = 0;
+        const Real eps_j = prj.z;
+        if (eps_j != 0) {
+            const Vec2<Real> se = sm.se[r];
+            const Real eps_i = se.b;
+            if (eps_i != 0) {
+                Real sig_grad, eps_grad;
+                lennard_jones<Real, U>(
+                    (Real)1, eps_i, eps_j, se.a, prj.y, inv_d, inv_d2, qij_inv, factor, erfc_bd, u, prefactor, sig_grad,
+                    eps_grad);
+                if (DP) {
+                    const Real ys = fmul(sig_grad, static_cast<Real>(FX_EXPONENT_SIG));
+                    const V2 ye = fmul2(
+                        fmul2(f2(eps_grad), make2(eps_j, eps_i)), f2(static_cast<Real>(FX_EXPONENT_EPS)));
+                    const unsigned long long gs = fixed_round(ys), ge = fixed_round(ye.x);
+                    g.sig += gs;
+                    g.eps += fixed_round(ye.y);
+                    constexpr int F = DX ? 3 : 0;
+                    if (fits_limbs(ys) && fits_limbs(ye.x)) {
+                        limbs_add(sm.acc, F + 1, copy + r, gs);
+                        limbs_add(sm.acc, F + 2, copy + r, ge);
+                    } else {
+                        red_add(out.sig + row_first + r, gs);
+                        red_add(out.eps + row_first + r, ge);
+                    }
+                }
+                if (DL && ALCH && INTERP) {
+                    real_du_dl = ffma(sig_grad, fadd(sm.dqs[r].b, dpj.y), real_du_dl);
+                    real_du_dl = ffma(eps_grad, sum_of_products_rn(eps_j, sm.de[r], eps_i, dpj.z), real_du_dl);
+                }
+            }
         }
-    }
-    if (DL && ALCH) {
-        real_du_dl = ffma(fmul(delta_w, prefactor), fsub(dw_dl_i, dw_dl_j), real_du_dl);
-        if (INTERP) {
-            real_du_dl = ffma(fmul(inv_d, erfc_bd), sum_of_products_rn(qj, dq_dl_i, qi, dq_dl_j), real_du_dl);
+        if (DX) {
+            const Real ex = static_cast<Real>(FX_EXPONENT);
+            const V2 yxy = fmul2(fmul2(f2(prefactor), dxy), f2(ex));
+            const Real yx = yxy.x, yy = yxy.y;
+            const Real yz = fmul(fmul(prefactor, delta_z), ex);
+            const unsigned long long fx = fixed_round(yx);
+            const unsigned long long fy = fixed_round(yy);
+            const unsigned long long fz = fixed_round(yz);
+            g.x -= fx;
+            g.y -= fy;
+            g.z -= fz;
+            if (fits_limbs(yx) && fits_limbs(yy) && fits_limbs(yz)) {
+                limbs_add(sm.acc, 0, copy + r, fx);
+                limbs_add(sm.acc, 1, copy + r, fy);
+                limbs_add(sm.acc, 2, copy + r, fz);
+            } else {
+                red_add(out.x + row_first + r, fx);
+                red_add(out.y + row_first + r, fy);
+                red_add(out.z + row_first + r, fz);
+                // llrint(-y) equals -llrint(y) except where the conversion
+                // saturates (|y| >= 2^63) or y is NaN: add the difference
+                if (!fixed_in_range(yx) || !fixed_in_range(yy) || !fixed_in_range(yz)) {
+                    g.x += fixed_round(-yx) + fx;
+                    g.y += fixed_round(-yy) + fy;
+                    g.z += fixed_round(-yz) + fz;
+                }
+            }
         }
-        du_dl += to_fixed(real_du_dl, FX_EXPONENT);
-    }
-    if (U) {
-        energy += to_fixed(u, FX_EXPONENT);
+        if (DP) {
+            const V2 yq = fmul2(
+                fmul2(fmul2(make2(qj, qi), f2(inv_d)), f2(erfc_bd)), f2(static_cast<Real>(FX_EXPONENT)));
+            const unsigned long long gq = fixed_round(yq.x);
+            g.q += fixed_round(yq.y);
+            constexpr int F = DX ? 3 : 0;
+            if (fits_limbs(yq.x)) {
+                limbs_add(sm.acc, F, copy + r, gq);
+            } else {
+                red_add(out.q + row_first + r, gq);
+            }
+        }
+        if (DL && ALCH) {
+            real_du_dl = ffma(fmul(delta_w, prefactor), fsub(dw_dl_i, prj.w), real_du_dl);
+            if (INTERP) {
+                real_du_dl =
+                    ffma(fmul(inv_d, erfc_bd), sum_of_products_rn(qj, sm.dqs[r].a, qi, dpj.x), real_du_dl);
+            }
+            g.dl += to_fixed(real_du_dl, FX_EXPONENT);
+        }
+        if (U) {
+            g.u += to_fixed(u, FX_EXPONENT);
+        }
     }
 }
 
-// One tile of RG rows x 32 columns: lane l owns row slot i (row l mod RG);
-// the column atoms rotate through the lanes of each RG-lane group by one
-// position per round (RG rounds), carrying their accumulators.
-// Per-pair arithmetic and validity follow
-// timemachine/cpp/src/kernels/k_nonbonded.cuh:424-546; the column
-// contribution of du_dx is the exact negation of the row contribution
-// (llrint is odd under round-half-even), so it is converted once.
-template <typename Real, bool U, bool DX, bool DL, bool DP, bool INTERP, bool ALCH, bool CHECK, int RG = TILE>
-__device__ __forceinline__ void sweep_tile(
+// One tile: column j of the lane (>= S: none) against the staged rows; the
+// columns' sums go to their accumulators.
+template <typename Real, bool U, bool DX, bool DL, bool DP, bool INTERP, int RG>
+__device__ __forceinline__ void walk_tile(
+    const PairArgs &a,
+    WalkRows<Real, DX, DP, INTERP, RG> &sm,
     const int lane,
-    const unsigned S,
-    const unsigned i,
-    unsigned j,
-    const Real ci_x,
-    const Real ci_y,
-    const Real ci_z,
-    const Real ci_w,
-    const Real qi,
-    const Real sig_i,
-    const Real eps_i,
-    const Real dw_dl_i,
-    const Real dq_dl_i,
-    const Real dsig_dl_i,
-    const Real deps_dl_i,
-    Real cj_x,
-    Real cj_y,
-    Real cj_z,
-    Real cj_w,
-    Real qj,
-    Real sig_j,
-    Real eps_j,
-    Real dw_dl_j,
-    Real dq_dl_j,
-    Real dsig_dl_j,
-    Real deps_dl_j,
-    const Real box_x,
-    const Real box_y,
-    const Real box_z,
-    const Real inv_box_x,
-    const Real inv_box_y,
-    const Real inv_box_z,
-    const Real cutoff_squared,
-    const Real beta,
-    unsigned long long &gi_x,
-    unsigned long long &gi_y,
-    unsigned long long &gi_z,
-    unsigned long long &g_qi,
-    unsigned long long &g_sigi,
-    unsigned long long &g_epsi,
-    unsigned long long &du_dl,
-    unsigned long long &energy,
-    unsigned long long &gj_x,
-    unsigned long long &gj_y,
-    unsigned long long &gj_z,
-    unsigned long long &g_qj,
-    unsigned long long &g_sigj,
-    unsigned long long &g_epsj) {
-    // rows of RG < 32 slots: the warp is 32/RG lane groups, each sweeping RG
-    // of the tile's columns against the RG rows (lane l holds row l mod RG), so
-    // the columns rotate inside their lane group and a tile takes RG rounds
-    const int src = (lane & ~(RG - 1)) | ((lane + 1) & (RG - 1));
-    // measured on B200: 4 rounds per iteration for the force-only variant,
-    // no unrolling for the variants with more outputs (register pressure)
-    constexpr int UNROLL = (DX && !U && !DL && !DP) ? 4 : 1;
-#pragma unroll UNROLL
-    for (int round = 0; round < RG; round++) {
-        Real delta_x, delta_y;
-        if constexpr (TMNB_PACKED_SCALAR && sizeof(Real) == 4) {
-            // x and y in the two components of one packed operation each
-            const float2 dxy = min_image2(
-                fsub2(make_float2(ci_x, ci_y), make_float2(cj_x, cj_y)), make_float2(-box_x, -box_y),
-                make_float2(inv_box_x, inv_box_y));
-            delta_x = dxy.x;
-            delta_y = dxy.y;
-        } else {
-            delta_x = min_image(fsub(ci_x, cj_x), box_x, inv_box_x);
-            delta_y = min_image(fsub(ci_y, cj_y), box_y, inv_box_y);
-        }
-        const Real delta_z = min_image(fsub(ci_z, cj_z), box_z, inv_box_z);
-        Real d2 = dist2(delta_x, delta_y, delta_z);
-        Real delta_w;
-        if (ALCH) {
-            delta_w = fsub(ci_w, cj_w);
-            d2 = add_w2(d2, delta_w);
-        }
-        // CHECK: the tile holds atoms of the row group itself, so i < j decides
-        // which lane evaluates each pair. Otherwise every column slot exceeds
-        // every row slot, and padding rows/columns carry NaN coordinates,
-        // which fail the cutoff test.
-        const bool valid = !CHECK || (i < S && j < S && i < j);
-        if (valid && d2 < cutoff_squared) {
-            pair_terms<Real, U, DX, DL, DP, INTERP, ALCH>(
-                delta_x, delta_y, delta_z, ALCH ? delta_w : (Real)0, d2, qi, sig_i, eps_i, dw_dl_i, dq_dl_i, dsig_dl_i,
-                deps_dl_i, qj, sig_j, eps_j, dw_dl_j, dq_dl_j, dsig_dl_j, deps_dl_j, beta, gi_x, gi_y, gi_z, g_qi,
-                g_sigi, g_epsi, du_dl, energy, gj_x, gj_y, gj_z, g_qj, g_sigj, g_epsj);
-        }
-        if (CHECK) {
-            j = __shfl_sync(FULL_MASK, j, src);
-        }
-        qj = __shfl_sync(FULL_MASK, qj, src);
-        eps_j = __shfl_sync(FULL_MASK, eps_j, src);
-        sig_j = __shfl_sync(FULL_MASK, sig_j, src);
-        cj_x = __shfl_sync(FULL_MASK, cj_x, src);
-        cj_y = __shfl_sync(FULL_MASK, cj_y, src);
-        cj_z = __shfl_sync(FULL_MASK, cj_z, src);
-        if (ALCH) {
-            cj_w = __shfl_sync(FULL_MASK, cj_w, src);
-            dw_dl_j = __shfl_sync(FULL_MASK, dw_dl_j, src);
-        }
+    const unsigned row_first,
+    const bool rows_alch,
+    const unsigned j,
+    const int window,
+    const WalkBox<Real> &b,
+    const Accum &out) {
+    using St = Staged<Real>;
+    using V = typename St::V;
+    const size_t wo = (size_t)window * a.S;
+    const bool col_ok = j < (unsigned)a.S;
+    const Real nan = static_cast<Real>(__int_as_float(0x7fffffff));
+    const V pwj = col_ok ? St::posw(a)[wo + j] : St::make(nan, nan, nan, 0);
+    const V prj = col_ok ? St::prm(a)[wo + j] : St::make(0, 0, 0, 0);
+    V dpj = St::make(0, 0, 0, 0);
+    if (INTERP && col_ok) {
+        dpj = St::dprm(a)[wo + j];
+    }
+    const bool alch = rows_alch || __any_sync(FULL_MASK, pwj.w != 0 || (INTERP && (dpj.x != 0 || dpj.y != 0 || dpj.z != 0)));
+    // Image count of the column against the rows. Subtraction, scaling and
+    // rounding are monotonic, so where the smallest and the largest row
+    // coordinate give the same count, every row between them does, and the
+    // column's image is one shift: -box * count (exact for counts up to 2) is
+    // what the general form's fused multiply-add adds.
+    const Real nx = round_half_even(fmul(fsub(sm.lo[0], pwj.x), b.inv_x));
+    const Real ny = round_half_even(fmul(fsub(sm.lo[1], pwj.y), b.inv_y));
+    const Real nz = round_half_even(fmul(fsub(sm.lo[2], pwj.z), b.inv_z));
+    const bool one_image = nx == round_half_even(fmul(fsub(sm.hi[0], pwj.x), b.inv_x)) &&
+                           ny == round_half_even(fmul(fsub(sm.hi[1], pwj.y), b.inv_y)) &&
+                           nz == round_half_even(fmul(fsub(sm.hi[2], pwj.z), b.inv_z)) && fabs(nx) <= 2 &&
+                           fabs(ny) <= 2 && fabs(nz) <= 2;
+    const bool wrap = __any_sync(FULL_MASK, col_ok && !one_image);
+    // a column of the row group itself pairs with the rows before it
+    const unsigned own = j - row_first;
+    const unsigned valid = !col_ok ? 0u : (own < (unsigned)RG ? (1u << own) - 1 : FULL_MASK);
+    ColSums g;
+#define TMB_WALK(ALCH_, WRAP_)                                                                                        \
+    walk_pairs<Real, U, DX, DL, DP, INTERP, ALCH_, WRAP_, RG>(                                                        \
+        sm, lane, row_first, valid, pwj, prj, dpj, fmul(-b.x, nx), fmul(-b.y, ny), fmul(-b.z, nz), b, out, g)
+    if (alch) {
+        TMB_WALK(true, true);
+    } else if (wrap) {
+        TMB_WALK(false, true);
+    } else {
+        TMB_WALK(false, false);
+    }
+#undef TMB_WALK
+    if (col_ok) {
         if (DX) {
-            gj_x = __shfl_sync(FULL_MASK, gj_x, src);
-            gj_y = __shfl_sync(FULL_MASK, gj_y, src);
-            gj_z = __shfl_sync(FULL_MASK, gj_z, src);
+            red_add(out.x + j, g.x);
+            red_add(out.y + j, g.y);
+            red_add(out.z + j, g.z);
         }
         if (DP) {
-            g_qj = __shfl_sync(FULL_MASK, g_qj, src);
-            g_sigj = __shfl_sync(FULL_MASK, g_sigj, src);
-            g_epsj = __shfl_sync(FULL_MASK, g_epsj, src);
+            red_add(out.q + j, g.q);
+            if (prj.z != 0) {
+                red_add(out.sig + j, g.sig);
+                red_add(out.eps + j, g.eps);
+            }
         }
-        if (DL && ALCH && INTERP) {
-            dsig_dl_j = __shfl_sync(FULL_MASK, dsig_dl_j, src);
-            deps_dl_j = __shfl_sync(FULL_MASK, deps_dl_j, src);
-            dq_dl_j = __shfl_sync(FULL_MASK, dq_dl_j, src);
+        if (DL && alch) {
+            red_add(out.dl + j, g.dl);
+        }
+        if (U) {
+            red_add(out.u + j, g.u);
         }
     }
+}
+
+// One work item: the tiles it.y .. it.y + it.z - 1 of row group it.x. With
+// skip_dep, tiles that hold a lambda-dependent atom are left out.
+template <typename Real, bool U, bool DX, bool DL, bool DP, bool INTERP, bool SKIP_DEP, int RG>
+__device__ __forceinline__ void walk_item(
+    const PairArgs &a,
+    WalkRows<Real, DX, DP, INTERP, RG> &sm,
+    const int lane,
+    const int4 it,
+    const int window,
+    const WalkBox<Real> &b,
+    const Accum &out) {
+    const unsigned row_first = (unsigned)(it.x * RG);
+    const unsigned i = row_first + (lane & (RG - 1));
+    if (SKIP_DEP && __any_sync(FULL_MASK, i < (unsigned)a.row_end && a.lamdep[i])) {
+        return; // evaluated per window by the (tile, window) units
+    }
+    const bool rows_alch = walk_load_rows(a, sm, lane, row_first, window);
+    for (int t = 0; t < it.z; t++) {
+        const unsigned j = a.tile_cols[((long long)it.y + t) * TILE + lane];
+        if (SKIP_DEP && __any_sync(FULL_MASK, j < (unsigned)a.S && a.lamdep[j])) {
+            continue;
+        }
+        walk_tile<Real, U, DX, DL, DP, INTERP, RG>(a, sm, lane, row_first, rows_alch, j, window, b, out);
+        if ((t + 1) % sm.FLUSH_TILES == 0 && t + 1 < it.z) {
+            walk_flush_rows(sm, lane, out, row_first, a.row_end);
+        }
+    }
+    walk_flush_rows(sm, lane, out, row_first, a.row_end);
 }
 
 // One scaled pair (exclusion / 1-4 correction), arithmetic of
@@ -1389,502 +1631,6 @@ __device__ __forceinline__ void scaled_pair(
     }
 }
 
-// One tile of a row group's rows (lane: row slot i) against the 32 column slots
-// j, for one window: load, sweep, column atomics. Row accumulators are
-// returned to the caller.
-template <typename Real, bool U, bool DX, bool DL, bool DP, bool INTERP, int RG = TILE>
-__device__ __forceinline__ void tile_pass(
-    const PairArgs &a,
-    const int lane,
-    const unsigned S,
-    const unsigned i,
-    const unsigned j,
-    const int window,
-    const Accum &acc_out,
-    const Real box_x,
-    const Real box_y,
-    const Real box_z,
-    const Real inv_box_x,
-    const Real inv_box_y,
-    const Real inv_box_z,
-    const Real cutoff_squared,
-    const Real beta,
-    unsigned long long &gi_x,
-    unsigned long long &gi_y,
-    unsigned long long &gi_z,
-    unsigned long long &g_qi,
-    unsigned long long &g_sigi,
-    unsigned long long &g_epsi,
-    unsigned long long &du_dl,
-    unsigned long long &energy) {
-    using St = Staged<Real>;
-    using V = typename St::V;
-    const size_t wo = (size_t)window * a.S;
-    const bool row_ok = i < (unsigned)a.row_end;
-    const bool col_ok = j < S;
-    const unsigned i_eff = row_ok ? i : 0xffffffffu; // invalid rows pair with nothing
-    // padding rows and columns: NaN coordinates (no pair passes the cutoff test), w = 0
-    const Real nan = static_cast<Real>(__int_as_float(0x7fffffff));
-    const V pwi = row_ok ? St::posw(a)[wo + i] : St::make(nan, nan, nan, 0);
-    const V pri = row_ok ? St::prm(a)[wo + i] : St::make(0, 0, 0, 0);
-    const V pwj = col_ok ? St::posw(a)[wo + j] : St::make(nan, nan, nan, 0);
-    const V prj = col_ok ? St::prm(a)[wo + j] : St::make(0, 0, 0, 0);
-    V dpi = St::make(0, 0, 0, 0);
-    V dpj = dpi;
-    if (INTERP) {
-        if (row_ok) {
-            dpi = St::dprm(a)[wo + i];
-        }
-        if (col_ok) {
-            dpj = St::dprm(a)[wo + j];
-        }
-    }
-    const bool row_alch = pwi.w != 0 || (INTERP && (dpi.x != 0 || dpi.y != 0 || dpi.z != 0));
-    const bool col_alch = pwj.w != 0 || (INTERP && (dpj.x != 0 || dpj.y != 0 || dpj.z != 0));
-    const bool alch = __any_sync(FULL_MASK, row_alch || col_alch);
-    unsigned long long gj_x = 0, gj_y = 0, gj_z = 0, g_qj = 0, g_sigj = 0, g_epsj = 0;
-    // Only a tile holding atoms of the row group itself (the diagonal block)
-    // needs the per-pair i < j test. The diagonal block is the first
-    // candidate of the list builder's first warp, so a full one fills a tile
-    // of its own; the flag is computed per tile either way.
-    const unsigned row_first = i & ~(unsigned)(RG - 1);
-    const bool check = __any_sync(FULL_MASK, col_ok && j < row_first + RG);
-#define TMB_SWEEP(ALCH_, CHECK_)                                                                                      \
-    sweep_tile<Real, U, DX, DL, DP, INTERP, ALCH_, CHECK_, RG>(                                                       \
-        lane, S, i_eff, j, pwi.x, pwi.y, pwi.z, pwi.w, pri.x, pri.y, pri.z, pri.w, dpi.x, dpi.y, dpi.z, pwj.x, pwj.y,   \
-        pwj.z, pwj.w, prj.x, prj.y, prj.z, prj.w, dpj.x, dpj.y, dpj.z, box_x, box_y, box_z, inv_box_x, inv_box_y,       \
-        inv_box_z, cutoff_squared, beta, gi_x, gi_y, gi_z, g_qi, g_sigi, g_epsi, du_dl, energy, gj_x, gj_y, gj_z, g_qj, \
-        g_sigj, g_epsj)
-    if (alch) {
-        if (check) {
-            TMB_SWEEP(true, true);
-        } else {
-            TMB_SWEEP(true, false);
-        }
-    } else {
-        if (check) {
-            TMB_SWEEP(false, true);
-        } else {
-            TMB_SWEEP(false, false);
-        }
-    }
-#undef TMB_SWEEP
-    if (col_ok) {
-        if (DX) {
-            red_add(acc_out.x + j, gj_x);
-            red_add(acc_out.y + j, gj_y);
-            red_add(acc_out.z + j, gj_z);
-        }
-        if (DP) {
-            red_add(acc_out.q + j, g_qj);
-            red_add(acc_out.sig + j, g_sigj);
-            red_add(acc_out.eps + j, g_epsj);
-        }
-    }
-}
-
-template <bool U, bool DX, bool DL, bool DP>
-__device__ __forceinline__ void flush_row(
-    const Accum &acc_out,
-    unsigned i,
-    unsigned long long gi_x,
-    unsigned long long gi_y,
-    unsigned long long gi_z,
-    unsigned long long g_qi,
-    unsigned long long g_sigi,
-    unsigned long long g_epsi,
-    unsigned long long du_dl,
-    unsigned long long energy) {
-    if (DX) {
-        red_add(acc_out.x + i, gi_x);
-        red_add(acc_out.y + i, gi_y);
-        red_add(acc_out.z + i, gi_z);
-    }
-    if (DP) {
-        red_add(acc_out.q + i, g_qi);
-        red_add(acc_out.sig + i, g_sigi);
-        red_add(acc_out.eps + i, g_epsi);
-    }
-    if (DL) {
-        red_add(acc_out.dl + i, du_dl);
-    }
-    if (U) {
-        red_add(acc_out.u + i, energy);
-    }
-}
-
-// Row sums of a tile sweep with RG-slot row groups: the 32/RG lanes holding
-// one row combine their partial sums, and the first of them flushes.
-template <int RG, bool U, bool DX, bool DL, bool DP>
-__device__ __forceinline__ void flush_row_rg(
-    const Accum &acc_out,
-    unsigned i,
-    bool row_ok,
-    unsigned long long gi_x,
-    unsigned long long gi_y,
-    unsigned long long gi_z,
-    unsigned long long g_qi,
-    unsigned long long g_sigi,
-    unsigned long long g_epsi,
-    unsigned long long du_dl,
-    unsigned long long energy) {
-    if (RG < TILE) {
-#pragma unroll
-        for (int o = RG; o < TILE; o <<= 1) {
-            if (DX) {
-                gi_x += __shfl_xor_sync(FULL_MASK, gi_x, o);
-                gi_y += __shfl_xor_sync(FULL_MASK, gi_y, o);
-                gi_z += __shfl_xor_sync(FULL_MASK, gi_z, o);
-            }
-            if (DP) {
-                g_qi += __shfl_xor_sync(FULL_MASK, g_qi, o);
-                g_sigi += __shfl_xor_sync(FULL_MASK, g_sigi, o);
-                g_epsi += __shfl_xor_sync(FULL_MASK, g_epsi, o);
-            }
-            if (DL) {
-                du_dl += __shfl_xor_sync(FULL_MASK, du_dl, o);
-            }
-            if (U) {
-                energy += __shfl_xor_sync(FULL_MASK, energy, o);
-            }
-        }
-        if ((threadIdx.x & (TILE - 1)) >= RG) {
-            return;
-        }
-    }
-    if (row_ok) {
-        flush_row<U, DX, DL, DP>(acc_out, i, gi_x, gi_y, gi_z, g_qi, g_sigi, g_epsi, du_dl, energy);
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Forces-only sweep with packed FP32 pairs (16-row tiles).
-//
-// sm_100 executes FP32x2 instructions (mul/add/sub/fma .rn.f32x2) whose two
-// components round exactly as the scalar __fmul_rn / __fadd_rn / __fsub_rn /
-// __fmaf_rn do. The forces-only sweep holds two rows per lane (rows r and
-// r + 8 of the 16-row group; the warp is four 8-lane groups, each rotating
-// its 8 columns through its lanes in 8 rounds) and evaluates the lane's two
-// pairs in the two components: the same per-pair roundings as pair_terms in
-// about half the FP32 instructions, and one column rotation for two pairs.
-// The transcendental steps (rsqrt, exp, the IEEE reciprocal) and the
-// fixed-point conversions stay per component, and the row and column forces
-// of a pair are converted once, as in pair_terms. The packed operations
-// (fmul2 and the others, nb_pair_math.cuh) are inline PTX, so a product
-// followed by a sum keeps both roundings. (The all-outputs variants keep the
-// one-row sweep: with two rows per lane they need 127 registers, 4 CTAs/SM,
-// and the 12-window call measured 2 % slower.)
-// ---------------------------------------------------------------------------
-// Row accumulators of the packed sweep: forces and energy.
-struct RowForces {
-    unsigned long long x = 0, y = 0, z = 0, u = 0;
-};
-
-// U: energy; DX: forces (one of them or both).
-template <bool U, bool DX, bool ALCH, bool CHECK>
-__device__ __forceinline__ void sweep_forces_p2(
-    const int lane,
-    const unsigned S,
-    const unsigned ia,
-    const unsigned ib,
-    unsigned j,
-    const float2 ci_x,
-    const float2 ci_y,
-    const float2 ci_z,
-    const float2 ci_w,
-    const float2 qi,
-    const float2 sig_i,
-    const float2 eps_i,
-    float cj_x,
-    float cj_y,
-    float cj_z,
-    float cj_w,
-    float qj,
-    float sig_j,
-    float eps_j,
-    const float2 neg_box_x,
-    const float2 neg_box_y,
-    const float2 neg_box_z,
-    const float2 inv_box_x,
-    const float2 inv_box_y,
-    const float2 inv_box_z,
-    const float cutoff_squared,
-    const float beta,
-    RowForces &A,
-    RowForces &B,
-    unsigned long long &gj_x,
-    unsigned long long &gj_y,
-    unsigned long long &gj_z) {
-    const int src = (lane & ~7) | ((lane + 1) & 7);
-#pragma unroll 1
-    for (int round = 0; round < 8; round++) {
-        const float2 dx = min_image2(fsub2(ci_x, f2(cj_x)), neg_box_x, inv_box_x);
-        const float2 dy = min_image2(fsub2(ci_y, f2(cj_y)), neg_box_y, inv_box_y);
-        const float2 dz = min_image2(fsub2(ci_z, f2(cj_z)), neg_box_z, inv_box_z);
-#if TMNB_DAG_D2 == 0
-        float2 d2 = ffma2(dz, dz, ffma2(dx, dx, fmul2(dy, dy)));
-#elif TMNB_DAG_D2 == 1
-        float2 d2 = ffma2(dz, dz, ffma2(dy, dy, fmul2(dx, dx)));
-#else
-        float2 d2 = fadd2(fadd2(fmul2(dx, dx), fmul2(dy, dy)), fmul2(dz, dz));
-#endif
-        if (ALCH) {
-            const float2 dw = fsub2(ci_w, f2(cj_w));
-            d2 = madd2(dw, dw, d2, TMNB_DAG_D4);
-        }
-        // validity as in sweep_tile
-        const bool in_a = (!CHECK || (ia < S && j < S && ia < j)) && d2.x < cutoff_squared;
-        const bool in_b = (!CHECK || (ib < S && j < S && ib < j)) && d2.y < cutoff_squared;
-        if (in_a || in_b) {
-            // electrostatics (nb_pair_math.cuh electrostatics / es_factor),
-            // charge scale 1
-            const float2 inv_d = make_float2(inv_sqrt(d2.x), inv_sqrt(d2.y));
-            const float2 d = fmul2(d2, inv_d);
-            const float2 inv_d2 = fmul2(inv_d, inv_d);
-            const float2 qij_inv = fmul2(fmul2(qi, f2(qj)), inv_d);
-            const float2 bd = fmul2(f2(beta), d);
-            const float2 bd2 = fmul2(bd, bd); // fmul(-bd, bd) == -(bd * bd)
-            const float2 e = make_float2(__expf(-bd2.x), __expf(-bd2.y));
-            const float2 den = madd2(f2(0.3275911f), bd, f2(1.0f), TMNB_DAG_DEN);
-            const float2 t = make_float2(__frcp_rn(den.x), __frcp_rn(den.y));
-            float2 poly = madd2(f2(1.061405429f), t, f2(-1.453152027f), TMNB_DAG_POLY);
-            poly = madd2(poly, t, f2(1.421413741f), TMNB_DAG_POLY);
-            poly = madd2(poly, t, f2(-0.284496736f), TMNB_DAG_POLY);
-            poly = madd2(poly, t, f2(0.254829592f), TMNB_DAG_POLY);
-            const float2 pt = fmul2(poly, t);
-            const float2 erfc_bd = fmul2(pt, e);
-            float2 pre = f2(0.0f);
-            if (DX) {
-                const float2 cbd = fmul2(f2(static_cast<float>(1.128379167095512595889238330988549829708)), bd);
-#if TMNB_DAG_ERF == 1
-                const float2 s = ffma2(cbd, e, erfc_bd);
-#elif TMNB_DAG_ERF == 0
-                const float2 s = fadd2(fmul2(cbd, e), erfc_bd);
-#else
-                const float2 s = ffma2(pt, e, fmul2(cbd, e));
-#endif
-                pre = fmul2(qij_inv, fmul2(make_float2(-inv_d2.x, -inv_d2.y), s));
-            }
-            float2 u = f2(0.0f);
-            if (U) {
-                u = fmul2(qij_inv, erfc_bd);
-            }
-            // Lennard-Jones where both atoms carry epsilon (per pair)
-            const bool lj_a = eps_i.x != 0 && eps_j != 0;
-            const bool lj_b = eps_i.y != 0 && eps_j != 0;
-            if ((in_a && lj_a) || (in_b && lj_b)) {
-                const float2 eps_ij = fmul2(eps_i, f2(eps_j));
-                const float2 sig_ij = fadd2(sig_i, f2(sig_j));
-                const float2 s1 = fmul2(sig_ij, inv_d);
-                const float2 s2 = fmul2(s1, s1);
-                const float2 s4 = fmul2(s2, s2);
-                const float2 s6 = fmul2(s4, s2);
-                if (DX) {
-                    const float2 ljx = fmul2(eps_ij, fmul2(s6, inv_d2));
-                    const float2 ljy = madd2(s6, f2(48.0f), f2(-24.0f), TMNB_DAG_LJP);
-#if TMNB_DAG_PRE == 1
-                    const float2 pre_lj = ffma2(make_float2(-ljx.x, -ljx.y), ljy, pre);
-#elif TMNB_DAG_PRE == 0
-                    const float2 pre_lj = fsub2(pre, fmul2(ljx, ljy));
-#else
-#error "TMNB_DAG_PRE == 2 has no packed form"
-#endif
-                    pre = make_float2(lj_a ? pre_lj.x : pre.x, lj_b ? pre_lj.y : pre.y);
-                }
-                if (U) {
-                    // lennard_jones of nb_pair_math.cuh: A = (4 eps_ij)(s6 - 1), u += A s6
-#if TMNB_DAG_S6M1
-                    const float2 s6m1 = ffma2(s4, s2, f2(-1.0f));
-#else
-                    const float2 s6m1 = fsub2(s6, f2(1.0f));
-#endif
-                    const float2 Acoef = fmul2(fmul2(f2(4.0f), eps_ij), s6m1);
-#if TMNB_DAG_U == 1
-                    const float2 u_lj = ffma2(Acoef, s6, u);
-#elif TMNB_DAG_U == 0
-                    const float2 u_lj = fadd2(u, fmul2(Acoef, s6));
-#else
-                    const float2 u_lj = ffma2(qij_inv, erfc_bd, fmul2(Acoef, s6));
-#endif
-                    u = make_float2(lj_a ? u_lj.x : u.x, lj_b ? u_lj.y : u.y);
-                }
-            }
-            if (U) {
-                const float2 yu = fmul2(u, f2(static_cast<float>(FX_EXPONENT)));
-                if (in_a) {
-                    A.u += fixed_round(yu.x);
-                }
-                if (in_b) {
-                    B.u += fixed_round(yu.y);
-                }
-            }
-            const float2 ex = f2(static_cast<float>(FX_EXPONENT));
-            const float2 yx = fmul2(fmul2(pre, dx), ex);
-            const float2 yy = fmul2(fmul2(pre, dy), ex);
-            const float2 yz = fmul2(fmul2(pre, dz), ex);
-            if (DX && in_a) {
-                const unsigned long long fx = fixed_round(yx.x), fy = fixed_round(yy.x), fz = fixed_round(yz.x);
-                A.x += fx;
-                A.y += fy;
-                A.z += fz;
-                gj_x -= fx;
-                gj_y -= fy;
-                gj_z -= fz;
-                if (!fixed_in_range(yx.x) || !fixed_in_range(yy.x) || !fixed_in_range(yz.x)) {
-                    gj_x += fixed_round(-yx.x) + fx;
-                    gj_y += fixed_round(-yy.x) + fy;
-                    gj_z += fixed_round(-yz.x) + fz;
-                }
-            }
-            if (DX && in_b) {
-                const unsigned long long fx = fixed_round(yx.y), fy = fixed_round(yy.y), fz = fixed_round(yz.y);
-                B.x += fx;
-                B.y += fy;
-                B.z += fz;
-                gj_x -= fx;
-                gj_y -= fy;
-                gj_z -= fz;
-                if (!fixed_in_range(yx.y) || !fixed_in_range(yy.y) || !fixed_in_range(yz.y)) {
-                    gj_x += fixed_round(-yx.y) + fx;
-                    gj_y += fixed_round(-yy.y) + fy;
-                    gj_z += fixed_round(-yz.y) + fz;
-                }
-            }
-        }
-        if (CHECK) {
-            j = __shfl_sync(FULL_MASK, j, src);
-        }
-        qj = __shfl_sync(FULL_MASK, qj, src);
-        eps_j = __shfl_sync(FULL_MASK, eps_j, src);
-        sig_j = __shfl_sync(FULL_MASK, sig_j, src);
-        cj_x = __shfl_sync(FULL_MASK, cj_x, src);
-        cj_y = __shfl_sync(FULL_MASK, cj_y, src);
-        cj_z = __shfl_sync(FULL_MASK, cj_z, src);
-        if (ALCH) {
-            cj_w = __shfl_sync(FULL_MASK, cj_w, src);
-        }
-        if (DX) {
-            gj_x = __shfl_sync(FULL_MASK, gj_x, src);
-            gj_y = __shfl_sync(FULL_MASK, gj_y, src);
-            gj_z = __shfl_sync(FULL_MASK, gj_z, src);
-        }
-    }
-}
-
-// One 16-row tile of a forces and / or energy evaluation (U, DX), window
-// `window`: the lane's rows ia and ia + 8 against column slot j.
-template <bool U, bool DX>
-__device__ __forceinline__ void tile_forces_p2(
-    const PairArgs &a,
-    const int lane,
-    const unsigned S,
-    const unsigned ia,
-    const unsigned j,
-    const int window,
-    const Accum &acc_out,
-    const float box_x,
-    const float box_y,
-    const float box_z,
-    const float inv_box_x,
-    const float inv_box_y,
-    const float inv_box_z,
-    const float cutoff_squared,
-    const float beta,
-    RowForces &A,
-    RowForces &B) {
-    const unsigned ib = ia + 8;
-    const size_t wo = (size_t)window * a.S;
-    const bool a_ok = ia < (unsigned)a.row_end;
-    const bool b_ok = ib < (unsigned)a.row_end;
-    const bool col_ok = j < S;
-    const float nan = __int_as_float(0x7fffffff);
-    const float4 pwa = a_ok ? a.posw[wo + ia] : make_float4(nan, nan, nan, 0.f);
-    const float4 pra = a_ok ? a.prm[wo + ia] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 pwb = b_ok ? a.posw[wo + ib] : make_float4(nan, nan, nan, 0.f);
-    const float4 prb = b_ok ? a.prm[wo + ib] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float4 pwj = col_ok ? a.posw[wo + j] : make_float4(nan, nan, nan, 0.f);
-    const float4 prj = col_ok ? a.prm[wo + j] : make_float4(0.f, 0.f, 0.f, 0.f);
-    // Forces and energies depend on the parameters' lambda derivatives only
-    // through w: a tile whose w are all zero adds dw*dw = 0 exactly, so it
-    // skips the 4th dimension whatever the interpolated parameters do.
-    const bool alch = __any_sync(FULL_MASK, pwa.w != 0.f || pwb.w != 0.f || pwj.w != 0.f);
-    const unsigned ia_eff = a_ok ? ia : 0xffffffffu;
-    const unsigned ib_eff = b_ok ? ib : 0xffffffffu;
-    const unsigned row_first = ia & ~15u;
-    const bool check = __any_sync(FULL_MASK, col_ok && j < row_first + 16);
-    unsigned long long gj_x = 0, gj_y = 0, gj_z = 0;
-#define TMB_SWEEP_P2(ALCH_, CHECK_)                                                                                    \
-    sweep_forces_p2<U, DX, ALCH_, CHECK_>(                                                                              \
-        lane, S, ia_eff, ib_eff, j, make_float2(pwa.x, pwb.x), make_float2(pwa.y, pwb.y), make_float2(pwa.z, pwb.z),   \
-        make_float2(pwa.w, pwb.w), make_float2(pra.x, prb.x), make_float2(pra.y, prb.y), make_float2(pra.z, prb.z),   \
-        pwj.x, pwj.y, pwj.z, pwj.w, prj.x, prj.y, prj.z, f2(-box_x), f2(-box_y), f2(-box_z), f2(inv_box_x),           \
-        f2(inv_box_y), f2(inv_box_z), cutoff_squared, beta, A, B, gj_x, gj_y, gj_z)
-    if (alch) {
-        if (check) {
-            TMB_SWEEP_P2(true, true);
-        } else {
-            TMB_SWEEP_P2(true, false);
-        }
-    } else {
-        if (check) {
-            TMB_SWEEP_P2(false, true);
-        } else {
-            TMB_SWEEP_P2(false, false);
-        }
-    }
-#undef TMB_SWEEP_P2
-    if (DX && col_ok) {
-        red_add(acc_out.x + j, gj_x);
-        red_add(acc_out.y + j, gj_y);
-        red_add(acc_out.z + j, gj_z);
-    }
-}
-
-// Row sums of a packed sweep: the four lanes holding rows ia / ia + 8
-// (lanes l, l^8, l^16, l^24) combine, and lanes 0-7 flush.
-template <bool U, bool DX>
-__device__ __forceinline__ void flush_forces_p2(const Accum &acc_out, unsigned ia, unsigned row_end, RowForces A,
-                                                RowForces B) {
-#pragma unroll
-    for (int o = 8; o < TILE; o <<= 1) {
-        if (DX) {
-            A.x += __shfl_xor_sync(FULL_MASK, A.x, o);
-            A.y += __shfl_xor_sync(FULL_MASK, A.y, o);
-            A.z += __shfl_xor_sync(FULL_MASK, A.z, o);
-            B.x += __shfl_xor_sync(FULL_MASK, B.x, o);
-            B.y += __shfl_xor_sync(FULL_MASK, B.y, o);
-            B.z += __shfl_xor_sync(FULL_MASK, B.z, o);
-        }
-        if (U) {
-            A.u += __shfl_xor_sync(FULL_MASK, A.u, o);
-            B.u += __shfl_xor_sync(FULL_MASK, B.u, o);
-        }
-    }
-    if ((threadIdx.x & (TILE - 1)) >= 8) {
-        return;
-    }
-    if (ia < row_end) {
-        if (DX) {
-            red_add(acc_out.x + ia, A.x);
-            red_add(acc_out.y + ia, A.y);
-            red_add(acc_out.z + ia, A.z);
-        }
-        if (U) {
-            red_add(acc_out.u + ia, A.u);
-        }
-    }
-    if (ia + 8 < row_end) {
-        if (DX) {
-            red_add(acc_out.x + ia + 8, B.x);
-            red_add(acc_out.y + ia + 8, B.y);
-            red_add(acc_out.z + ia + 8, B.z);
-        }
-        if (U) {
-            red_add(acc_out.u + ia + 8, B.u);
-        }
-    }
-}
-
 // Multi-window calls: lists the tiles with at least one lambda-dependent row
 // or column atom (the tiles the pair kernel evaluates once per window). One
 // warp per work item, grid-stride.
@@ -1924,6 +1670,28 @@ static __global__ void k_dep_tiles(DepArgs a, DevState *state) {
     }
 }
 
+// The warp's next work unit: n_first + the counter's value.
+__device__ __forceinline__ int next_unit(int *counter, int n_first, int lane) {
+    int v = 0;
+    if (lane == 0) {
+        v = atomicAdd(counter, 1);
+    }
+    return n_first + __shfl_sync(FULL_MASK, v, 0);
+}
+
+// CTAs per SM the compiler must fit for each pair-kernel variant (its
+// register budget).
+template <typename Real, bool U, bool DX, bool DL, bool DP, bool INTERP, int RG>
+constexpr int pair_min_ctas() {
+    if (sizeof(Real) != 4) {
+        return TMNB_WALK_CTAS_F64;
+    }
+    if (DP) {
+        return TMNB_WALK_CTAS_ALL;
+    }
+    return TMNB_WALK_CTAS;
+}
+
 // Persistent pair kernel over dynamically scheduled work units:
 //   [0, n_items)                 tile work items (row group, first tile, count);
 //   MULTI only: [n_items, + n_dep*K)  one lambda-dependent tile at one window;
@@ -1931,48 +1699,17 @@ static __global__ void k_dep_tiles(DepArgs a, DevState *state) {
 // MULTI (K > 1 windows): the tile items skip lambda-dependent tiles and add
 // into the shared accumulator block; each (tile, window) unit adds into the
 // window's block; a lambda-dependent scaled pair is evaluated for every window.
-// CTAs per SM the compiler must fit for each pair-kernel variant (its
-// register budget): measured on B200, see the kernel below.
-template <typename Real, bool U, bool DX, bool DL, bool DP, bool INTERP, int RG>
-constexpr int pair_min_ctas() {
-    if (sizeof(Real) != 4) {
-        return 5;
-    }
-    if (U && DX && DL && DP && !INTERP) {
-        return 6;
-    }
-    if (DX && !U && !DL && !DP) {
-        return (TMNB_PACKED_FORCES && RG == 16) ? TMNB_PACKED_FORCES_CTAS : 8;
-    }
-    if (U && !DX && !DL && !DP && TMNB_PACKED_FORCES && TMNB_PACKED_ENERGY && RG == 16) {
-        return TMNB_PACKED_FORCES_CTAS;
-    }
-    return 1;
-}
-
 template <typename Real, bool U, bool DX, bool DL, bool DP, bool INTERP, bool MULTI, int RG = TILE>
-// Occupancy, measured on B200: all four outputs at 6 CTAs/SM (80 registers,
-// no spills; 12-window call -3.5 % against 5); forces only or energy only
-// with the packed two-rows sweep at 6 (80), forces only with 8 or 32 rows per
-// tile at 8 (64). FP64
-// variants at 5 (96 registers, a few spilled words): the 12-window call
-// took 0.407 ms against 0.455 ms at the compiler's 154 registers (3 CTAs).
 __global__ void __launch_bounds__(128, (pair_min_ctas<Real, U, DX, DL, DP, INTERP, RG>())) k_pair(PairArgs a) {
+    __shared__ WalkRows<Real, DX, DP, INTERP, RG> rows[4];
     grid_dependency_wait();
     if (a.state->error) {
         return;
     }
     const int lane = threadIdx.x & 31;
-    const Real box_x = a.box[0 * 3 + 0];
-    const Real box_y = a.box[1 * 3 + 1];
-    const Real box_z = a.box[2 * 3 + 2];
-    const Real inv_box_x = 1 / box_x;
-    const Real inv_box_y = 1 / box_y;
-    const Real inv_box_z = 1 / box_z;
-    const Real real_cutoff = static_cast<Real>(a.cutoff);
-    const Real cutoff_squared = real_cutoff * real_cutoff;
-    const Real beta = static_cast<Real>(a.beta);
-    const unsigned S = (unsigned)a.S;
+    WalkRows<Real, DX, DP, INTERP, RG> &sm = rows[threadIdx.x >> 5];
+    walk_clear(sm, lane);
+    const WalkBox<Real> b = walk_box<Real>(a.box, a.cutoff, a.beta);
     const int n_items = a.state->n_items;
     const int n_dep_units = MULTI ? a.state->n_dep * a.K : 0;
     if (MULTI && blockIdx.x == 0 && threadIdx.x == 0 && !a.state->error) {
@@ -1982,19 +1719,13 @@ __global__ void __launch_bounds__(128, (pair_min_ctas<Real, U, DX, DL, DP, INTER
     }
     const int n_tiles_units = n_items + n_dep_units;
     const int n_total = n_tiles_units + (a.M + TILE - 1) / TILE;
-    // forces-only FP32 evaluations of 16-row tiles take the packed sweep
-    constexpr bool PACKED =
-        TMNB_PACKED_FORCES && sizeof(Real) == 4 && RG == 16 && !DL && !DP && ((DX && !U) || (U && !DX && TMNB_PACKED_ENERGY));
 
-    for (;;) {
-        int item = 0;
-        if (lane == 0) {
-            item = atomicAdd(&a.state->next_item, 1);
-        }
-        item = __shfl_sync(FULL_MASK, item, 0);
-        if (item >= n_total) {
-            break;
-        }
+    // the first unit of a warp is its own number, the others come from the
+    // counter: thousands of warps asking for their first one at once (and, in
+    // a small system, for a second one that does not exist) wait for one another
+    const int n_warps = gridDim.x * (blockDim.x / TILE);
+    for (int item = (blockIdx.x * blockDim.x + threadIdx.x) / TILE; item < n_total;
+         item = next_unit(&a.state->next_item, n_warps, lane)) {
         if (item >= n_tiles_units) {
             const int pair = (item - n_tiles_units) * TILE + lane;
             if (pair < a.M) {
@@ -2002,82 +1733,28 @@ __global__ void __launch_bounds__(128, (pair_min_ctas<Real, U, DX, DL, DP, INTER
                 const int atom_j = a.pair_idxs[2 * pair + 1];
                 const int si = a.slot_of ? a.slot_of[atom_i] : atom_i;
                 const int sj = a.slot_of ? a.slot_of[atom_j] : atom_j;
-                if (!MULTI || !(a.lamdep[si] || a.lamdep[sj])) {
+                const bool dep = MULTI && (a.lamdep[si] || a.lamdep[sj]);
+                for (int k = 0; k < (dep ? a.K : 1); k++) {
                     scaled_pair<Real, U, DX, DL, DP, INTERP>(
-                        a, pair, si, sj, 0, a.acc, box_x, box_y, box_z, inv_box_x, inv_box_y, inv_box_z,
-                        cutoff_squared);
-                } else {
-                    for (int k = 0; k < a.K; k++) {
-                        scaled_pair<Real, U, DX, DL, DP, INTERP>(
-                            a, pair, si, sj, k, acc_block(a.acc, a.acc_block, 1 + k), box_x, box_y, box_z, inv_box_x,
-                            inv_box_y, inv_box_z, cutoff_squared);
-                    }
+                        a, pair, si, sj, k, acc_block(a.acc, a.acc_block, dep ? 1 + k : 0), b.x, b.y, b.z, b.inv_x,
+                        b.inv_y, b.inv_z, b.cutoff_squared);
                 }
             }
             continue;
         }
-        if constexpr (PACKED) {
-            // two rows per lane: ia and ia + 8 of the 16-row group
-            if (MULTI && item >= n_items) {
-                const int unit = item - n_items;
-                const int2 dt = a.dep_tiles[unit / a.K];
-                const int k = unit % a.K;
-                const unsigned ia = (unsigned)(dt.x * RG + (lane & 7));
-                const unsigned j = a.tile_cols[(long long)dt.y * TILE + lane];
-                const Accum wk = acc_block(a.acc, a.acc_block, 1 + k);
-                RowForces A, B;
-                tile_forces_p2<U, DX>(a, lane, S, ia, j, k, wk, box_x, box_y, box_z, inv_box_x, inv_box_y, inv_box_z,
-                               cutoff_squared, beta, A, B);
-                flush_forces_p2<U, DX>(wk, ia, (unsigned)a.row_end, A, B);
-                continue;
-            }
-            const int4 it = a.items[item];
-            const unsigned ia = (unsigned)(it.x * RG + (lane & 7));
-            const bool row_dep = MULTI && ((ia < (unsigned)a.row_end && a.lamdep[ia]) ||
-                                           (ia + 8 < (unsigned)a.row_end && a.lamdep[ia + 8]));
-            RowForces A, B;
-            for (int t = 0; t < it.z; t++) {
-                const long long tile = (long long)it.y + t;
-                const unsigned j = a.tile_cols[tile * TILE + lane];
-                if (MULTI && __any_sync(FULL_MASK, row_dep || (j < S && a.lamdep[j]))) {
-                    continue; // evaluated per window by the (tile, window) units
-                }
-                tile_forces_p2<U, DX>(a, lane, S, ia, j, 0, a.acc, box_x, box_y, box_z, inv_box_x, inv_box_y, inv_box_z,
-                               cutoff_squared, beta, A, B);
-            }
-            flush_forces_p2<U, DX>(a.acc, ia, (unsigned)a.row_end, A, B);
-            continue;
-        }
+        int4 it;
+        int window = 0;
         if (MULTI && item >= n_items) {
             const int unit = item - n_items;
             const int2 dt = a.dep_tiles[unit / a.K];
-            const int k = unit % a.K;
-            const unsigned i = (unsigned)(dt.x * RG + (lane & (RG - 1)));
-            const unsigned j = a.tile_cols[(long long)dt.y * TILE + lane];
-            const Accum wk = acc_block(a.acc, a.acc_block, 1 + k);
-            unsigned long long wx = 0, wy = 0, wz = 0, wq = 0, ws = 0, we = 0, wl = 0, wu = 0;
-            tile_pass<Real, U, DX, DL, DP, INTERP, RG>(
-                a, lane, S, i, j, k, wk, box_x, box_y, box_z, inv_box_x, inv_box_y, inv_box_z, cutoff_squared, beta,
-                wx, wy, wz, wq, ws, we, wl, wu);
-            flush_row_rg<RG, U, DX, DL, DP>(wk, i, i < (unsigned)a.row_end, wx, wy, wz, wq, ws, we, wl, wu);
+            window = unit % a.K;
+            it = make_int4(dt.x, dt.y, 1, 0);
+            walk_item<Real, U, DX, DL, DP, INTERP, false, RG>(
+                a, sm, lane, it, window, b, acc_block(a.acc, a.acc_block, 1 + window));
             continue;
         }
-        const int4 it = a.items[item];
-        const unsigned i = (unsigned)(it.x * RG + (lane & (RG - 1)));
-        const bool row_dep = MULTI && i < (unsigned)a.row_end && a.lamdep[i];
-        unsigned long long gi_x = 0, gi_y = 0, gi_z = 0, g_qi = 0, g_sigi = 0, g_epsi = 0, du_dl = 0, energy = 0;
-        for (int t = 0; t < it.z; t++) {
-            const long long tile = (long long)it.y + t;
-            const unsigned j = a.tile_cols[tile * TILE + lane];
-            if (MULTI && __any_sync(FULL_MASK, row_dep || (j < S && a.lamdep[j]))) {
-                continue; // evaluated per window by the (tile, window) units
-            }
-            tile_pass<Real, U, DX, DL, DP, INTERP, RG>(
-                a, lane, S, i, j, 0, a.acc, box_x, box_y, box_z, inv_box_x, inv_box_y, inv_box_z, cutoff_squared,
-                beta, gi_x, gi_y, gi_z, g_qi, g_sigi, g_epsi, du_dl, energy);
-        }
-        flush_row_rg<RG, U, DX, DL, DP>(
-            a.acc, i, i < (unsigned)a.row_end, gi_x, gi_y, gi_z, g_qi, g_sigi, g_epsi, du_dl, energy);
+        it = a.items[item];
+        walk_item<Real, U, DX, DL, DP, INTERP, MULTI, RG>(a, sm, lane, it, 0, b, a.acc);
     }
 }
 

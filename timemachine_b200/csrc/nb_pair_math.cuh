@@ -156,6 +156,21 @@ __device__ __forceinline__ float2 madd2(float2 a, float2 b, float2 c, int fused)
     return fused ? ffma2(a, b, c) : fadd2(fmul2(a, b), c);
 }
 
+// The same operations on two FP64 values (two scalar instructions each), so
+// that the tile walk is written once for both arithmetic types.
+__device__ __forceinline__ double2 f2(double v) { return make_double2(v, v); }
+__device__ __forceinline__ double2 fmul2(double2 a, double2 b) { return make_double2(fmul(a.x, b.x), fmul(a.y, b.y)); }
+__device__ __forceinline__ double2 fadd2(double2 a, double2 b) { return make_double2(fadd(a.x, b.x), fadd(a.y, b.y)); }
+__device__ __forceinline__ double2 fsub2(double2 a, double2 b) { return make_double2(fsub(a.x, b.x), fsub(a.y, b.y)); }
+__device__ __forceinline__ double2 ffma2(double2 a, double2 b, double2 c) {
+    return make_double2(ffma(a.x, b.x, c.x), ffma(a.y, b.y, c.y));
+}
+__device__ __forceinline__ double2 madd2(double2 a, double2 b, double2 c, int fused) {
+    return fused ? ffma2(a, b, c) : fadd2(fmul2(a, b), c);
+}
+__device__ __forceinline__ float2 make2(float a, float b) { return make_float2(a, b); }
+__device__ __forceinline__ double2 make2(double a, double b) { return make_double2(a, b); }
+
 // a*b + c*d with both products rounded before the sum.
 template <typename Real> __device__ __forceinline__ Real sum_of_products_rn(Real a, Real b, Real c, Real d) {
     return fadd(fmul(a, b), fmul(c, d));
@@ -207,6 +222,19 @@ template <typename Real> __device__ __forceinline__ Real add_w2(Real d2, Real dw
 #endif
 }
 
+// dist2 of two pairs
+template <typename V2> __device__ __forceinline__ V2 dist2_of_two(V2 dx, V2 dy, V2 dz) {
+#if TMNB_DAG_D2 == 0
+    return ffma2(dz, dz, ffma2(dx, dx, fmul2(dy, dy)));
+#elif TMNB_DAG_D2 == 1
+    return ffma2(dz, dz, ffma2(dy, dy, fmul2(dx, dx)));
+#else
+    return fadd2(fadd2(fmul2(dx, dx), fmul2(dy, dy)), fmul2(dz, dz));
+#endif
+}
+__device__ __forceinline__ float2 dist2(float2 dx, float2 dy, float2 dz) { return dist2_of_two(dx, dy, dz); }
+__device__ __forceinline__ double2 dist2(double2 dx, double2 dy, double2 dz) { return dist2_of_two(dx, dy, dz); }
+
 // min_image per component; neg_box = -box.
 __device__ __forceinline__ float2 min_image2(float2 delta, float2 neg_box, float2 inv_box) {
     const float2 magic = f2(12582912.0f); // round_half_even
@@ -216,6 +244,10 @@ __device__ __forceinline__ float2 min_image2(float2 delta, float2 neg_box, float
 #else
     return fadd2(delta, fmul2(neg_box, n));
 #endif
+}
+
+__device__ __forceinline__ double2 min_image2(double2 delta, double2 neg_box, double2 inv_box) {
+    return make_double2(min_image(delta.x, -neg_box.x, inv_box.x), min_image(delta.y, -neg_box.y, inv_box.y));
 }
 
 template <typename Real> __device__ __forceinline__ Real madd(Real a, Real b, Real c, int fused) {

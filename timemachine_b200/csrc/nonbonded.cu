@@ -24,15 +24,6 @@
 #include <string>
 #include <vector>
 
-// Tiles per work item of lists built by single-window calls.
-#ifndef TMNB_SINGLE_CHUNK
-#define TMNB_SINGLE_CHUNK 2
-#endif
-// Tiles per work item of lists built by multi-window calls.
-#ifndef TMNB_MULTI_CHUNK
-#define TMNB_MULTI_CHUNK 4
-#endif
-
 namespace tmb {
 
 enum class Kind { AllPairs, PairList, Nonbonded, Group };
@@ -408,6 +399,22 @@ class NonbondedPotential : public PotentialBase {
         return L;
     }
 
+    // Tiles per work item of a list built by a K-window call: few enough that
+    // every resident warp has work and the last items end together, as many as
+    // that allows (each item loads and flushes its rows once). Measured on B200,
+    // us per call, 1 / 2 / 4 tiles (forces) and 2 / 4 / 8 (12 windows):
+    // 2,500 atoms 26.1 / 30.8 / 40.2 and 53.0 / 64.2 / 86.5; 10,000: 46.5 / 48.7 /
+    // 55.0 and 83.3 / 87.0 / 101; 22,840: 81.2 / 79.6 / 84.8 and 136.1 / 137.2 /
+    // 147; 98,000: 273 / 252 / 249 and 455 / 436 / 441.
+    int list_chunk(int K) const {
+        // a group's rows reach about twice the columns of as many all-pairs rows
+        const long long n = kind_ == Kind::Group ? 2LL * NR_ : S_;
+        if (K > 1) {
+            return n < 4000 ? 1 : (n < 40000 ? 2 : 4);
+        }
+        return n < 16000 ? 1 : 2;
+    }
+
     int row_end() const { return kind_ == Kind::Group ? NR_ : S_; }
 
     // Elements of one accumulator block (8 or 11 arrays of S slots).
@@ -688,19 +695,17 @@ class NonbondedPotential : public PotentialBase {
         ta.n_row_blocks = n_row_blocks_;
         ta.cb_first = cb_first_;
         ta.radius = (float)(cutoff_ + padding_ + 1e-5);
+        ta.cutoff = (float)cutoff_;
         ta.box = d_box;
         ta.posw = posw_.p;
         ta.prm = prm_.p;
+        ta.lamdep = lamdep_.p;
         ta.bb_ctr = bb_ctr_.p;
         ta.bb_ext = bb_ext_.p;
         ta.tile_cols = tile_cols_.p;
         ta.rb_ntiles = rb_ntiles_.p;
         ta.items = items_.p;
-        // tiles per work item, measured on B200 at 22,840 atoms: two for a
-        // single window with the packed forces sweep (MD step 125.7 -> 121.3
-        // us against one; one had been -8 % against four with the one-row
-        // sweep), four for several windows (fewer row flushes: -3 %)
-        ta.chunk = K > 1 ? TMNB_MULTI_CHUNK : TMNB_SINGLE_CHUNK;
+        ta.chunk = list_chunk(K);
         const DevState *cst = state_.p;
         launch_dependent(k_bin_keys, dim3(sgrid), dim3(tpb), 0, stream, sa, cst);
         launch_dependent(k_bin_scan, dim3(1), dim3(1024), 0, stream, sa, state_.p);

@@ -373,6 +373,86 @@ __device__ __forceinline__ void lennard_jones(
     eps_grad = fmul(fmul(fmul(lj_scale, (Real)4), s6m1), s6);
 }
 
+// es_factor and lennard_jones (scales 1) of two FP32 pairs.
+__device__ __forceinline__ float2 es_factor2(float beta, float2 d, float2 inv_d2, float2 &erfc_bd) {
+    const float2 bd = fmul2(f2(beta), d);
+    const float2 bd2 = fmul2(bd, bd); // fmul(-bd, bd) == -(bd * bd)
+    const float2 e = make_float2(__expf(-bd2.x), __expf(-bd2.y));
+    const float2 den = madd2(f2(0.3275911f), bd, f2(1.0f), TMNB_DAG_DEN);
+    const float2 t = make_float2(__frcp_rn(den.x), __frcp_rn(den.y));
+    float2 poly = madd2(f2(1.061405429f), t, f2(-1.453152027f), TMNB_DAG_POLY);
+    poly = madd2(poly, t, f2(1.421413741f), TMNB_DAG_POLY);
+    poly = madd2(poly, t, f2(-0.284496736f), TMNB_DAG_POLY);
+    poly = madd2(poly, t, f2(0.254829592f), TMNB_DAG_POLY);
+    const float2 pt = fmul2(poly, t);
+    erfc_bd = fmul2(pt, e);
+    const float2 cbd = fmul2(f2(static_cast<float>(1.128379167095512595889238330988549829708)), bd);
+#if TMNB_DAG_ERF == 1
+    const float2 s = ffma2(cbd, e, erfc_bd);
+#elif TMNB_DAG_ERF == 0
+    const float2 s = fadd2(fmul2(cbd, e), erfc_bd);
+#else
+    const float2 s = ffma2(pt, e, fmul2(cbd, e));
+#endif
+    return fmul2(make_float2(-inv_d2.x, -inv_d2.y), s);
+}
+
+template <bool COMPUTE_U>
+__device__ __forceinline__ void lennard_jones2(
+    const float2 eps_i,
+    const float2 eps_j,
+    const float2 sig_i,
+    const float2 sig_j,
+    const float2 inv_d,
+    const float2 inv_d2,
+    const float2 qij_inv,
+    const float2 factor,
+    const float2 erfc_bd,
+    float2 &u,
+    float2 &prefactor,
+    float2 &sig_grad,
+    float2 &eps_grad) {
+    const float2 eps_ij = fmul2(eps_i, eps_j);
+    const float2 sig_ij = fadd2(sig_i, sig_j);
+    const float2 s1 = fmul2(sig_ij, inv_d);
+    const float2 s2 = fmul2(s1, s1);
+    const float2 s4 = fmul2(s2, s2);
+    const float2 s6 = fmul2(s4, s2);
+    const float2 s5_inv_d = fmul2(fmul2(sig_ij, s4), inv_d2);
+#if TMNB_DAG_S6M1
+    const float2 s6m1 = ffma2(s4, s2, f2(-1.0f));
+#else
+    const float2 s6m1 = fsub2(s6, f2(1.0f));
+#endif
+    const float2 ljx = fmul2(eps_ij, fmul2(s6, inv_d2));
+    const float2 ljy = madd2(s6, f2(48.0f), f2(-24.0f), TMNB_DAG_LJP);
+#if TMNB_DAG_PRE == 1
+    prefactor = ffma2(make_float2(-ljx.x, -ljx.y), ljy, prefactor);
+#elif TMNB_DAG_PRE == 0
+    prefactor = fsub2(prefactor, fmul2(ljx, ljy));
+#else
+    const float2 ljxy = fmul2(ljx, ljy);
+    prefactor = ffma2(qij_inv, factor, make_float2(-ljxy.x, -ljxy.y));
+#endif
+    if (COMPUTE_U) {
+        const float2 A = fmul2(fmul2(f2(4.0f), eps_ij), s6m1);
+#if TMNB_DAG_U == 1
+        u = ffma2(A, s6, u);
+#elif TMNB_DAG_U == 0
+        u = fadd2(u, fmul2(A, s6));
+#else
+        u = ffma2(qij_inv, erfc_bd, fmul2(A, s6));
+#endif
+    }
+#if TMNB_DAG_2S6M1
+    const float2 two_s6_m1 = fsub2(ffma2(s4, s2, s6), f2(1.0f));
+#else
+    const float2 two_s6_m1 = ffma2(f2(2.0f), s6, f2(-1.0f));
+#endif
+    sig_grad = fmul2(fmul2(fmul2(f2(24.0f), eps_ij), s5_inv_d), two_s6_m1);
+    eps_grad = fmul2(fmul2(f2(4.0f), s6m1), s6);
+}
+
 // Neighbour-list validity: true when an atom moved more than half the padding
 // since the last rebuild (squared displacement against (padding / 2)^2).
 // Explicit rounding, so the pair kernel's own check and the MD integrator's

@@ -1,4 +1,4 @@
-"""The tile walk of the pair kernel against the pair-list kernel over the same
+"""The tile walk of the pair kernel, and the list rebuild before it, against the pair-list kernel over the same
 pairs: every output is an exact integer sum of per-pair fixed-point values, and
 both kernels round a pair the same way, so they agree bit for bit. Sizes sit at
 the edges of tiles and row groups; coordinates lie in several periodic images
@@ -8,6 +8,7 @@ column buffer."""
 
 import numpy as np
 import pytest
+from scipy.spatial import cKDTree
 
 from tests.helpers import f32_round, random_params
 from timemachine_b200 import potentials as P
@@ -89,3 +90,31 @@ def test_dense_group_fills_the_column_buffer(interpolated):
     got = [np.sort(t) for t in tiles]
     assert max(len(t) for t in got) > 3072
     assert all(len(np.unique(t)) == len(t) for t in got)
+
+
+@pytest.mark.parametrize("n", [255, 8192, 8193, 32768, 32769])
+def test_rebuild_paths(n):
+    """Sizes at the edges of the three ways a call prepares and sorts: the list
+    that each leaves gives the pair list's sums, with and without the Hilbert
+    order, after the atoms have moved and with other windows per call."""
+    rng = np.random.default_rng(n)
+    edge = max(2.0, (n / 100.0) ** (1.0 / 3.0))
+    cutoff, beta = 0.4, 2.0
+    box = np.eye(3) * edge
+    p = f32_round(random_params(rng, n))
+    plane, offset = np.zeros(n, np.int32), (rng.random(n) < 0.002).astype(np.int32)
+    impl = P.NonbondedAllPairs(plane, offset, beta, cutoff).unbound_impl(np.float32)
+    plain = P.NonbondedAllPairs(plane, offset, beta, cutoff).unbound_impl(np.float32)
+    plain.disable_hilbert_sort()
+    for _ in range(2):
+        x = f32_round(rng.uniform(0, edge, size=(n, 3)))
+        wrapped = np.minimum(x - edge * np.floor(x / edge), np.nextafter(edge, 0))
+        pairs = cKDTree(wrapped, boxsize=edge).query_pairs(cutoff + 1e-3, output_type="ndarray").astype(np.int32)
+        ref = P.NonbondedPairList(pairs, np.ones((len(pairs), 2)), plane, offset, beta, cutoff).unbound_impl(np.float32)
+        want = _fixed(ref, x, p, box, 0.3)
+        _assert_same(_fixed(impl, x, p, box, 0.3), want)
+        _assert_same(_fixed(plain, x, p, box, 0.3), want)
+    multi = impl.execute_windows_fixed(x, p, box, np.array([0.3, 0.9]))
+    _assert_same([multi[k][0] if k < 2 else multi[k][0].sum(dtype=np.uint64) for k in range(4)], want)
+    energy = _fixed(impl, x, p, box, 0.3, (False, False, False, True))
+    _assert_same(energy, want)

@@ -175,7 +175,7 @@ __global__ void k_b_scatter(const Rep *__restrict__ reps, const int2 *__restrict
 }
 
 // Lennard-Jones atoms first within the replica's 32-slot block rb (one warp),
-// as lj_first_warp does for a single system; restages the moved slots.
+// as stage_block does for a single system; restages the moved slots.
 __device__ __forceinline__ void lj_first_rep(const Rep &r, int rb) {
     const int lane = threadIdx.x & 31;
     const int lo = rb * TILE;
@@ -214,7 +214,10 @@ __global__ void k_b_bounds(const Rep *__restrict__ reps, const int2 *__restrict_
         return;
     }
     lj_first_rep(r, m.y);
-    block_bounds_warp(r.N, m.y, r.box, r.posw, r.bb_ctr, r.bb_ext);
+    const int s = m.y * TILE + (int)(threadIdx.x & 31);
+    const bool valid = s < r.N;
+    block_bounds_warp(
+        valid, valid ? r.posw[s] : make_float4(0.f, 0.f, 0.f, 0.f), r.box, m.y, r.bb_ctr, r.bb_ext);
 }
 
 // Exclusive prefix over replicas of count(replica) into prefix[0..R-1], the

@@ -85,9 +85,9 @@ __global__ void k_langevin(
 // The integrator step fused with a potential's per-step staging and force
 // scatter (MDFusion). Each atom's force adds the potential's slot-ordered
 // fixed-point accumulator (what k_finalize would have added; integer sums, so
-// the order does not matter); a memset after the kernel clears the
-// accumulators for the next step (clearing each slot here, from the gathered
-// reads, measured slower). With `stage_next` the
+// the order does not matter); the next step's tile-build launch clears the
+// accumulators (clearing each slot here, from the gathered reads, measured
+// slower). With `stage_next` the
 // new coordinates are staged into the potential's slots and the
 // neighbour-list test of k_check_prepare is taken, so the next step's forces
 // start at the rebuild chain and the pair kernel.
@@ -557,7 +557,6 @@ class Context {
                 (const double *)cbs_.p, (const double *)ccs_.p, dt_, x_.p, v_.p, du_dx_.p, key_, st_.p, f,
                 stage_next ? 1 : 0);
             CK(cudaPeekAtLastError());
-            CK(cudaMemsetAsync(f.acc, 0, 3 * (size_t)f.S * sizeof(unsigned long long), stream_));
             return;
         }
         launch_dependent(

@@ -5,13 +5,17 @@
 //                     changed), box validation, and the per-slot FP32 staging
 //                     of coordinates, w, parameters (and dp/dlambda) using the
 //                     current slot order.
-//   k_bin_keys / k_bin_scan / k_bin_scatter / k_block_bounds / k_build_tiles
-//                     neighbour-list rebuild; every one returns at once unless
-//                     the rebuild flag is set, so the sequence is graph-capturable.
+//   k_order_slots / k_stage_blocks / k_build_tiles
+//                     neighbour-list rebuild: slot order, staging of the new
+//                     order, tiles; every one returns at once unless the
+//                     rebuild flag is set, so the sequence is graph-capturable.
+//                     k_build_tiles clears the accumulators in any case.
+//                     (k_prepare_sort: the whole front of a small system's call;
+//                     k_bin_keys / k_bin_scan / k_bin_scatter: the order of many atoms.)
 //   k_pair            persistent kernel over the tile work items and the
 //                     exclusion / scaled-pair chunks (dynamic scheduling).
 //   k_finalize        scatter of the slot-ordered int64 accumulators into the
-//                     caller's original-order outputs, then zeroing.
+//                     caller's original-order outputs.
 //
 // The work of each stage follows the reference pipeline
 // (timemachine/cpp/src/nonbonded_all_pairs.cu:222-433,
@@ -192,14 +196,15 @@ __device__ __forceinline__ void prepare_slot(const PrepareArgs &a, int s, int at
 // ---------------------------------------------------------------------------
 // Rebuild decision + staging.
 // ---------------------------------------------------------------------------
-static __global__ void k_check_prepare(
-    PrepareArgs a,
-    const unsigned *__restrict__ perm, // [S] slot -> atom
-    const double *__restrict__ nb_x,   // [N,3] coordinates at the last rebuild (nullptr: no neighbour list)
-    const double *__restrict__ nb_box, // [9]
-    DevState *state) {
-    grid_dependency_wait();
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+// The work of thread tid of n_threads.
+__device__ __forceinline__ void check_prepare(
+    const PrepareArgs &a,
+    const unsigned *perm, // [S] slot -> atom
+    const double *nb_x,   // [N,3] coordinates at the last rebuild (nullptr: no neighbour list)
+    const double *nb_box, // [9]
+    DevState *state,
+    const int tid,
+    const int n_threads) {
     if (tid == 0) {
         state->next_item = 0;
         if (nb_x != nullptr) {
@@ -232,7 +237,7 @@ static __global__ void k_check_prepare(
     // the rebuild test and the slot's lambda dependence
     const double half_pad2 = 0.25 * a.padding * a.padding;
     const size_t total = (size_t)a.S * (size_t)a.K;
-    for (size_t t = tid; t < total; t += (size_t)gridDim.x * blockDim.x) {
+    for (size_t t = tid; t < total; t += n_threads) {
         const int k = (int)(t / (size_t)a.S);
         const int s = (int)(t - (size_t)k * a.S);
         const int atom = perm[s];
@@ -258,6 +263,17 @@ static __global__ void k_check_prepare(
             state->n_dep = 0;
         }
     }
+}
+
+static __global__ void k_check_prepare(
+    PrepareArgs a,
+    const unsigned *__restrict__ perm,
+    const double *__restrict__ nb_x,
+    const double *__restrict__ nb_box,
+    DevState *state) {
+    grid_dependency_wait();
+    check_prepare(
+        a, perm, nb_x, nb_box, state, blockIdx.x * blockDim.x + threadIdx.x, (int)(gridDim.x * blockDim.x));
 }
 
 // ---------------------------------------------------------------------------
@@ -438,98 +454,31 @@ __device__ __forceinline__ int scatter_slot(
     return s;
 }
 
-static __global__ void k_bin_scatter(
-    SortArgs sa,
-    PrepareArgs pa,
-    unsigned *__restrict__ perm,    // [S] slot -> atom
-    int *__restrict__ slot_of,      // [N] atom -> slot (nullptr: not needed)
-    double *__restrict__ nb_x,      // [N,3]
-    double *__restrict__ nb_box,    // [9]
-    const DevState *state) {
+// Slot order after the counting sort (cells in Hilbert order, arbitrary within
+// a cell), or the set order without the sort.
+__device__ __forceinline__ void order_slot(const SortArgs &sa, int k, unsigned *perm) {
+    perm[sa.hilbert ? atomicAdd(&sa.bin_cursor[sa.keys[k]], 1) : k] = (unsigned)set_atom(sa, k);
+}
+
+static __global__ void k_bin_scatter(SortArgs sa, unsigned *perm, const DevState *state) {
     grid_dependency_wait();
     if (!state->rebuild || state->error) {
         return;
     }
-    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (tid < 9) {
-        nb_box[tid] = sa.box[tid];
-    }
-    for (int k = tid; k < sa.S; k += gridDim.x * blockDim.x) {
-        const int atom = set_atom(sa, k);
-        const int s = scatter_slot(sa, k, perm, slot_of, nb_x);
-        prepare_slot(pa, s, atom);
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < sa.S; k += gridDim.x * blockDim.x) {
+        order_slot(sa, k, perm);
     }
 }
 
-// ---------------------------------------------------------------------------
-// Block bounding boxes: one warp per 32-slot block; every atom is imaged
-// next to the block's first atom, then min/max give centre and half-extent.
-// ---------------------------------------------------------------------------
 __device__ __forceinline__ float wrap_delta(float d, float L, float inv_L) { return d - L * rintf(d * inv_L); }
 
-// Lennard-Jones atoms first within each row group (`rows` slots) of the
-// 32-slot block rb (one warp): the pair kernel's LJ branch is taken in a
-// rotation round only when some lane pairs two LJ atoms, and with LJ rows and
-// LJ columns both leading the tile those pairs fall in fewer rounds. Sorting
-// within row groups, not across them, keeps each group spatially compact.
-// Blocks that straddle the interaction group's row/column boundary keep their
-// order. Restages the moved atoms' slots.
-__device__ __forceinline__ void lj_first_warp(
-    const PrepareArgs &pa, int S, int n_first, int rb, unsigned *__restrict__ perm, int *__restrict__ slot_of,
-    int rows = TILE) {
-    const int lane = threadIdx.x & 31;
-    const int lo = rb * TILE;
-    const int hi = min(S, lo + TILE);
-    if (lo < n_first && hi > n_first) {
-        return;
-    }
-    const int s = lo + lane;
-    const bool valid = s < S;
-    const unsigned atom = valid ? perm[s] : 0u;
-    bool lj = false;
-    if (valid) {
-        lj = pa.p[3 * (size_t)atom + 2] != 0.0;
-        if (pa.interpolated) {
-            lj = lj || pa.p[3 * ((size_t)pa.N + atom) + 2] != 0.0;
-        }
-    }
-    const unsigned m = __ballot_sync(FULL_MASK, lj);
-    const unsigned vm = __ballot_sync(FULL_MASK, valid);
-    if (m == 0u || m == vm) {
-        return;
-    }
-    const unsigned lt = (1u << lane) - 1u;
-    const int seg = lane / rows;
-    const unsigned segm = (rows == TILE ? FULL_MASK : ((1u << rows) - 1u)) << (seg * rows);
-    const int pos = seg * rows +
-                    (lj ? __popc(m & lt & segm) : __popc(m & segm) + __popc(vm & ~m & lt & segm));
-    __syncwarp();
-    if (valid && lo + pos != s) {
-        const int ns = lo + pos;
-        perm[ns] = atom;
-        if (slot_of) {
-            slot_of[atom] = ns;
-        }
-        prepare_slot(pa, ns, (int)atom);
-    }
-    __syncwarp();
-}
-
-// Bounding box of the 32-slot block rb (one warp).
+// Bounding box of the 32-slot block rb (one warp) from its atoms' positions p.
 __device__ __forceinline__ void block_bounds_warp(
-    int S,
-    int rb,
-    const double *__restrict__ box,
-    const float4 *__restrict__ posw,
-    float4 *__restrict__ bb_ctr,
-    float4 *__restrict__ bb_ext) {
+    const bool valid, const float4 p, const double *box, int rb, float4 *bb_ctr, float4 *bb_ext) {
     const int lane = threadIdx.x & 31;
     const float Lx = (float)box[0], Ly = (float)box[4], Lz = (float)box[8];
     const float iLx = 1.0f / Lx, iLy = 1.0f / Ly, iLz = 1.0f / Lz;
     {
-        const int s = rb * TILE + lane;
-        const bool valid = s < S;
-        float4 p = valid ? posw[s] : make_float4(0.f, 0.f, 0.f, 0.f);
         const float rx = __shfl_sync(FULL_MASK, p.x, 0);
         const float ry = __shfl_sync(FULL_MASK, p.y, 0);
         const float rz = __shfl_sync(FULL_MASK, p.z, 0);
@@ -558,26 +507,139 @@ __device__ __forceinline__ void block_bounds_warp(
     }
 }
 
-static __global__ void k_block_bounds(
-    int S,
-    const double *__restrict__ box,
-    const float4 *__restrict__ posw,
-    float4 *__restrict__ bb_ctr,
-    float4 *__restrict__ bb_ext,
-    const DevState *state,
-    PrepareArgs pa,
-    int n_first,
-    unsigned *__restrict__ perm,
-    int *__restrict__ slot_of,
-    int rows) {
+struct SortTargets {
+    unsigned *perm; // [S] slot -> atom
+    int *slot_of;   // [N] atom -> slot (nullptr: not needed)
+    double *nb_x;   // [N,3] coordinates of the rebuild
+    double *nb_box; // [9]
+    float4 *bb_ctr, *bb_ext;
+    int rows;
+};
+
+// The new slot order's 32-slot block rb (one warp): Lennard-Jones atoms first
+// within each row group (`rows` slots), then the atoms' staging, the rebuild's
+// coordinates and the block's bounding box. With LJ rows first and LJ columns
+// in tiles of their own the pair kernel's LJ part runs in fewer steps; sorting
+// within row groups, not across them, keeps each group spatially compact.
+// Blocks that straddle the interaction group's row/column boundary keep their
+// order.
+__device__ __forceinline__ void stage_block(
+    const SortArgs &sa, const PrepareArgs &pa, const SortTargets &to, const int rb) {
+    const int lane = threadIdx.x & 31;
+    const int s = rb * TILE + lane;
+    const bool valid = s < sa.S;
+    const unsigned atom = valid ? to.perm[s] : 0u;
+    bool lj = false;
+    if (valid) {
+        lj = pa.p[3 * (size_t)atom + 2] != 0.0;
+        if (pa.interpolated) {
+            lj = lj || pa.p[3 * ((size_t)pa.N + atom) + 2] != 0.0;
+        }
+    }
+    const unsigned m = __ballot_sync(FULL_MASK, lj);
+    const unsigned vm = __ballot_sync(FULL_MASK, valid);
+    int pos = lane;
+    if (!(rb * TILE < sa.n_first && min(sa.S, rb * TILE + TILE) > sa.n_first)) {
+        const unsigned lt = (1u << lane) - 1u;
+        const int seg = lane / to.rows;
+        const unsigned segm = (to.rows == TILE ? FULL_MASK : ((1u << to.rows) - 1u)) << (seg * to.rows);
+        pos = seg * to.rows + (lj ? __popc(m & lt & segm) : __popc(m & segm) + __popc(vm & ~m & lt & segm));
+    }
+    __syncwarp(); // every lane has read its slot
+    float4 at = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (valid) {
+        const int ns = rb * TILE + pos;
+        to.perm[ns] = atom;
+        if (to.slot_of) {
+            to.slot_of[atom] = ns;
+        }
+        const double *xa = pa.x + 3 * (size_t)atom;
+        at = make_float4((float)xa[0], (float)xa[1], (float)xa[2], 0.f);
+        for (int d = 0; d < 3; d++) {
+            to.nb_x[3 * (size_t)atom + d] = xa[d];
+        }
+        prepare_slot(pa, ns, (int)atom);
+    }
+    block_bounds_warp(valid, at, sa.box, rb, to.bb_ctr, to.bb_ext);
+}
+
+static __global__ void k_stage_blocks(SortArgs sa, PrepareArgs pa, SortTargets to, const DevState *state) {
     grid_dependency_wait();
     if (!state->rebuild || state->error) {
         return;
     }
-    const int RB = (S + TILE - 1) / TILE;
-    for (int rb = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; rb < RB; rb += (gridDim.x * blockDim.x) >> 5) {
-        lj_first_warp(pa, S, n_first, rb, perm, slot_of, rows);
-        block_bounds_warp(S, rb, box, posw, bb_ctr, bb_ext);
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    if (tid < 9) {
+        to.nb_box[tid] = sa.box[tid];
+    }
+    const int RB = (sa.S + TILE - 1) / TILE;
+    for (int rb = tid >> 5; rb < RB; rb += (gridDim.x * blockDim.x) >> 5) {
+        stage_block(sa, pa, to, rb);
+    }
+}
+
+// The slot order (keys, scan, scatter) by one cluster of CTAs with hardware
+// barriers between the phases: one launch instead of three, which every call
+// that does not rebuild pays for too. Eight SMs are enough for a few ten
+// thousand atoms (NonbondedPotential::CLUSTER_SORT_MAX).
+constexpr int SORT_CTAS = 8; // the portable cluster size
+constexpr int SORT_THREADS = 1024;
+
+// Barrier of the cluster; global memory written before it is visible after it.
+__device__ __forceinline__ void cluster_barrier() {
+    __threadfence();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ void order_slots_cluster(const SortArgs &sa, unsigned *perm, DevState *state) {
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int T = SORT_CTAS * SORT_THREADS;
+    if (sa.hilbert) {
+        for (int k = tid; k < sa.S; k += T) {
+            bin_key(sa, k);
+        }
+    }
+    cluster_barrier();
+    if (blockIdx.x == 0) {
+        bin_scan_cta(sa, state);
+    }
+    cluster_barrier();
+    for (int k = tid; k < sa.S; k += T) {
+        order_slot(sa, k, perm);
+    }
+}
+
+static __global__ void __cluster_dims__(SORT_CTAS, 1, 1) __launch_bounds__(SORT_THREADS, 1)
+    k_order_slots(SortArgs sa, unsigned *perm, DevState *state) {
+    grid_dependency_wait();
+    if (!state->rebuild || state->error) { // the same for every CTA: nothing here changes them
+        return;
+    }
+    order_slots_cluster(sa, perm, state);
+}
+
+// Rebuild decision and staging (k_check_prepare), and where a rebuild is due
+// the sort and the new order's staging, by the same cluster: one launch for the
+// whole front of a small system's call.
+static __global__ void __cluster_dims__(SORT_CTAS, 1, 1) __launch_bounds__(SORT_THREADS, 1)
+    k_prepare_sort(SortArgs sa, PrepareArgs pa, SortTargets to, DevState *state) {
+    grid_dependency_wait();
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+    check_prepare(pa, to.perm, to.nb_x, to.nb_box, state, tid, SORT_CTAS * SORT_THREADS);
+    cluster_barrier();
+    const volatile DevState *now = state;
+    if (!now->rebuild || now->error) {
+        return;
+    }
+    order_slots_cluster(sa, to.perm, state);
+    cluster_barrier();
+    if (tid < 9) {
+        to.nb_box[tid] = sa.box[tid];
+    }
+    const int RB = (sa.S + TILE - 1) / TILE;
+    for (int rb = tid >> 5; rb < RB; rb += (SORT_CTAS * SORT_THREADS) >> 5) {
+        stage_block(sa, pa, to, rb);
     }
 }
 
@@ -968,9 +1030,15 @@ __device__ __forceinline__ void build_tiles_cta(const TileArgs &a, const int rb,
     }
 }
 
-static __global__ void __launch_bounds__(TB_WARPS * 32, TMNB_TB_CTAS) k_build_tiles(TileArgs a, DevState *state) {
+static __global__ void __launch_bounds__(TB_WARPS * 32, TMNB_TB_CTAS) k_build_tiles(
+    TileArgs a, unsigned long long *clear, size_t n_clear, DevState *state) {
     grid_dependency_wait();
-    if (!state->rebuild || state->error) {
+    // the accumulators the pair kernel adds into, cleared in this launch
+    // instead of one of its own
+    for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n_clear; k += (size_t)gridDim.x * blockDim.x) {
+        clear[k] = 0;
+    }
+    if (!state->rebuild || state->error || (int)blockIdx.x >= a.n_row_blocks) {
         return;
     }
     build_tiles_cta(a, blockIdx.x, state);
@@ -1883,7 +1951,7 @@ __global__ void __launch_bounds__(128, (pair_min_ctas<Real, U, DX, DL, DP, INTER
 
 // ---------------------------------------------------------------------------
 // Scatter of the slot-ordered accumulators into the caller's outputs (which
-// accumulate, +=), and reset of the accumulators. Window k's result is the
+// accumulate, +=). Window k's result is the
 // shared block plus block 1 + k (one window: block 0 only).
 // du_dp of interpolated potentials is split into the lambda=0 and lambda=1
 // halves per potential part, with the rounding of
@@ -1923,10 +1991,9 @@ __device__ __forceinline__ unsigned long long take(unsigned long long *p) {
 // One thread per (window k, set atom), consecutive threads on consecutive
 // atoms, so the output updates are coalesced and the slot-ordered
 // accumulators are gathered through slot_of. Only the accumulators of
-// requested outputs are read (the others were never written and stay zero).
-// take = 1 zeroes each accumulator after the read (one window: every slot is
-// read by exactly one thread); otherwise the caller zeroes the accumulator
-// blocks after this kernel. Outputs are added with integer atomics, so other
+// requested outputs are read (the others are not cleared and may hold an
+// earlier call's sums). take = 1 zeroes each accumulator after the read (one
+// window: every slot is read by exactly one thread). Outputs are added with integer atomics, so other
 // potentials may accumulate into the same buffers concurrently (the sums are
 // order-independent).
 static __global__ void k_finalize(FinalizeArgs a) {

@@ -216,9 +216,9 @@ class NonbondedPotential : public PotentialBase {
     }
 
     // CUDA events around every stage of a call (on the launching stream):
-    // TMNB_STAGE_PREPARE (k_check_prepare), _REBUILD (the five rebuild-chain
-    // kernels, which return at once when no rebuild is due), _PAIR (k_pair),
-    // _FINALIZE (k_finalize and the accumulator memset).
+    // TMNB_STAGE_PREPARE (k_check_prepare), _REBUILD (the rebuild-chain
+    // kernels, which return at once when no rebuild is due, and the clearing of
+    // the accumulators), _PAIR (k_pair), _FINALIZE (k_finalize).
     void enable_timing(bool on) {
         if (on && !timing_) {
             for (auto &e : ev_) {
@@ -399,6 +399,18 @@ class NonbondedPotential : public PotentialBase {
         return L;
     }
 
+    // Atoms up to which the slot order is computed by one cluster of 8 CTAs, and
+    // staged slots (atoms x windows) up to which that cluster takes the rebuild
+    // decision and the staging too. Each launch left out saves a call about 1.3
+    // us; eight SMs then limit a rebuild. Measured on B200, us per forces call
+    // without / with a rebuild: 2,500 atoms three launches more 29.0 / 53.0, one
+    // cluster 23.4 / 54.6; 10,000 atoms 46.4 / 83.6, order only 42.2 / 83.1,
+    // everything 45.2 / 94.1; 22,840 atoms 77.2 / 135.8, order only 72.2 / 137.1,
+    // everything 78.1 / 156.2; 98,000 atoms three kernels 242.0 / 429.3, order in
+    // the cluster 240.3 / 461.0.
+    static constexpr int CLUSTER_SORT_MAX = 32768;
+    static constexpr long long CLUSTER_PREPARE_MAX = 8192;
+
     // Tiles per work item of a list built by a K-window call: few enough that
     // every resident warp has work and the last items end together, as many as
     // that allows (each item loads and flushes its rows once). Measured on B200,
@@ -534,7 +546,11 @@ class NonbondedPotential : public PotentialBase {
         // k_check_prepare: one thread per (window, slot)
         const int pgrid = (int)std::max<size_t>(
             1, std::min<size_t>(((size_t)S_ * K + tpb - 1) / tpb, 8 * (size_t)num_sms()));
-        if (!(fuse_ & FUSE_PRESTAGED)) {
+        const int kidx = (d_du_dp ? 1 : 0) | (d_du_dl ? 2 : 0) | (d_du_dx ? 4 : 0) | (d_u ? 8 : 0);
+        const bool prestaged = fuse_ & FUSE_PRESTAGED;
+        // one kernel for the decision, the staging and the sort
+        const bool one_front = has_nblist_ && !prestaged && !timing_ && (long long)S_ * K <= CLUSTER_PREPARE_MAX;
+        if (!prestaged && !one_front) {
             stage_begin(TMNB_STAGE_PREPARE, stream);
             launch_dependent(
                 k_check_prepare, dim3(pgrid), dim3(tpb), 0, stream, pa, (const unsigned *)perm_.p,
@@ -544,11 +560,10 @@ class NonbondedPotential : public PotentialBase {
         }
         if (has_nblist_) {
             stage_begin(TMNB_STAGE_REBUILD, stream);
-            record_rebuild_chain(d_x, d_box, pa, sgrid, tpb, stream, K);
+            record_rebuild_chain(d_x, d_box, pa, sgrid, tpb, stream, K, one_front, kidx);
             stage_end(TMNB_STAGE_REBUILD, stream);
         }
 
-        const int kidx = (d_du_dp ? 1 : 0) | (d_du_dl ? 2 : 0) | (d_du_dx ? 4 : 0) | (d_u ? 8 : 0);
         if (kidx != 0 && K > 1 && has_nblist_) {
             DepArgs da;
             da.S = S_;
@@ -627,12 +642,10 @@ class NonbondedPotential : public PotentialBase {
             stage_begin(TMNB_STAGE_FINALIZE, stream);
             launch_dependent(k_finalize, dim3(fgrid), dim3(tpb), 0, stream, fa);
             CK(cudaPeekAtLastError());
-            // Zero the accumulator blocks k_finalize read (one coalesced memset;
-            // zeroing each slot as it is read, from k_finalize's gathered
-            // accesses, measured 2.5x slower). Forces only: the first three
-            // arrays of the block are the only ones written.
-            const size_t used = (kidx == 4 && K == 1) ? 3 * (size_t)S_ : acc_block_elems() * (K > 1 ? 1 + K : 1);
-            CK(cudaMemsetAsync(acc_.p, 0, used * sizeof(unsigned long long), stream));
+            if (!has_nblist_) { // else k_build_tiles clears them before the pair kernel
+                CK(cudaMemsetAsync(
+                    acc_.p, 0, acc_block_elems() * (K > 1 ? 1 + K : 1) * sizeof(unsigned long long), stream));
+            }
             stage_end(TMNB_STAGE_FINALIZE, stream);
         }
     }
@@ -672,7 +685,8 @@ class NonbondedPotential : public PotentialBase {
     // Neighbour-list rebuild: spatial sort (keys, scan, scatter), block
     // bounds, tile build. Each kernel returns at once unless state->rebuild.
     void record_rebuild_chain(
-        const double *d_x, const double *d_box, const PrepareArgs &pa, int sgrid, int tpb, cudaStream_t stream, int K) {
+        const double *d_x, const double *d_box, const PrepareArgs &pa, int sgrid, int tpb, cudaStream_t stream, int K,
+        bool one_front, int kidx) {
         SortArgs sa;
         sa.N = N_;
         sa.S = S_;
@@ -707,15 +721,43 @@ class NonbondedPotential : public PotentialBase {
         ta.items = items_.p;
         ta.chunk = list_chunk(K);
         const DevState *cst = state_.p;
-        launch_dependent(k_bin_keys, dim3(sgrid), dim3(tpb), 0, stream, sa, cst);
-        launch_dependent(k_bin_scan, dim3(1), dim3(1024), 0, stream, sa, state_.p);
+        SortTargets to;
+        to.perm = perm_.p;
+        to.slot_of = slot_of_.p;
+        to.nb_x = nb_x_.p;
+        to.nb_box = nb_box_.p;
+        to.bb_ctr = bb_ctr_.p;
+        to.bb_ext = bb_ext_.p;
+        to.rows = rows_;
+        if (one_front) {
+            launch_dependent(k_prepare_sort, dim3(SORT_CTAS), dim3(SORT_THREADS), 0, stream, sa, pa, to, state_.p);
+        } else {
+            if (S_ <= CLUSTER_SORT_MAX) {
+                launch_dependent(k_order_slots, dim3(SORT_CTAS), dim3(SORT_THREADS), 0, stream, sa, perm_.p, state_.p);
+            } else {
+                launch_dependent(k_bin_keys, dim3(sgrid), dim3(tpb), 0, stream, sa, cst);
+                launch_dependent(k_bin_scan, dim3(1), dim3(1024), 0, stream, sa, state_.p);
+                launch_dependent(k_bin_scatter, dim3(sgrid), dim3(tpb), 0, stream, sa, perm_.p, cst);
+            }
+            launch_dependent(
+                k_stage_blocks, dim3((RB_ + 3) / 4), dim3(128), 0, stream, sa, pa, to, cst);
+        }
+        // the accumulators this call adds into: the arrays of its outputs (one
+        // window: x y z, q sig eps, u, dl, then the scaled pairs' q sig eps)
+        size_t first = 0, last = acc_block_elems() * (K > 1 ? 1 + K : 1);
+        if (K == 1) {
+            const size_t S = S_;
+            first = (kidx & 4) ? 0 : (kidx & 1) ? 3 * S : (kidx & 8) ? 6 * S : 7 * S;
+            last = (kidx & 1) && split_pair_dp_ ? 11 * S
+                                                : (kidx & 2) ? 8 * S : (kidx & 8) ? 7 * S : (kidx & 1) ? 6 * S : 3 * S;
+        }
+        const size_t n_clear = kidx == 0 ? 0 : last - first;
+        // one CTA per row group; more where few row groups (an interaction
+        // group's) would clear for long
+        const size_t ctas = std::max<size_t>(
+            n_row_blocks_, std::min<size_t>(num_sms(), (n_clear + TB_WARPS * 32 - 1) / (TB_WARPS * 32)));
         launch_dependent(
-            k_bin_scatter, dim3(sgrid), dim3(tpb), 0, stream, sa, pa, perm_.p, slot_of_.p, nb_x_.p, nb_box_.p, cst);
-        const int bb_grid = std::max(1, (RB_ * 32 + tpb - 1) / tpb);
-        launch_dependent(
-            k_block_bounds, dim3(bb_grid), dim3(tpb), 0, stream, S_, d_box, (const float4 *)posw_.p, bb_ctr_.p,
-            bb_ext_.p, cst, pa, sa.n_first, perm_.p, slot_of_.p, rows_);
-        launch_dependent(k_build_tiles, dim3(n_row_blocks_), dim3(TB_WARPS * 32), 0, stream, ta, state_.p);
+            k_build_tiles, dim3((unsigned)ctas), dim3(TB_WARPS * 32), 0, stream, ta, acc_.p + first, n_clear, state_.p);
         CK(cudaPeekAtLastError());
     }
 

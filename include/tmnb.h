@@ -471,6 +471,22 @@ tmnb_status tmnb_potential_adjoint_device(
     double *d_grad_w, /* [N] += */
     void *stream);
 
+/* tmnb_potential_adjoint_device with the upstream gradient of du_dl read from
+ * device memory when the kernel runs, so the caller need not wait for it. */
+tmnb_status tmnb_potential_adjoint_device_all(
+    tmnb_potential *pot,
+    int N,
+    int P,
+    const double *d_x,
+    const double *d_p,
+    const double *d_box,
+    double lambda,
+    const double *d_g_du_dx, /* [N,3] */
+    const double *d_g_du_dl, /* one value */
+    double *d_grad_p,        /* [N,3], += */
+    double *d_grad_w,        /* [N], += */
+    void *stream);
+
 /*
  * Replica batch (no single reference counterpart: it replaces the loops in
  * which the reference evaluates or simulates replicas one at a time, one

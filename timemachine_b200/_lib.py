@@ -158,6 +158,8 @@ def _declare(lib):
     lib.tmnb_potential_nblist_rows.restype = ctypes.c_int
     lib.tmnb_potential_adjoint_device.argtypes = [vp, i, i, vp, vp, vp, d, vp, d, vp, vp, vp]
     lib.tmnb_potential_adjoint_device.restype = ctypes.c_int
+    lib.tmnb_potential_adjoint_device_all.argtypes = [vp, i, i, vp, vp, vp, d, vp, vp, vp, vp, vp]
+    lib.tmnb_potential_adjoint_device_all.restype = ctypes.c_int
     lib.tmnb_batch_create.argtypes = [ctypes.POINTER(vp)]
     lib.tmnb_batch_destroy.argtypes = [vp]
     lib.tmnb_batch_add.argtypes = [vp, i, vp, vp, vp, vp, vp, vp, i, vp, vp, i, vp, vp, i, vp, vp, d, d, d, d, d, vp, vp,

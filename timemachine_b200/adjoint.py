@@ -37,7 +37,7 @@ class NonbondedForces(torch.autograd.Function):
         p, x, box = ctx.saved_tensors
         N = x.shape[0]
         g_dx = torch.zeros((N, 3), dtype=torch.float64, device=x.device) if g_dx is None else g_dx.contiguous()
-        g_dl = 0.0 if g_dl is None else float(g_dl)
+        g_dl = 0.0 if g_dl is None else g_dl  # a device value is read by the kernel, not waited for
         grad_p = torch.zeros(p.numel(), dtype=torch.float64, device=x.device)
         grad_w = torch.zeros(N, dtype=torch.float64, device=x.device)
         ctx.impl.adjoint_device(x, p.reshape(-1), box, ctx.lam, g_dx.to(torch.float64), g_dl, grad_p, grad_w)

@@ -850,6 +850,7 @@ class NonbondedPotential : public PotentialBase {
         double lambda,
         const double *d_g_dx,
         double g_dl,
+        const double *d_g_dl, // nullptr: g_dl
         double *d_grad_p,
         double *d_grad_w,
         cudaStream_t stream) {
@@ -878,19 +879,20 @@ class NonbondedPotential : public PotentialBase {
         a.perm = perm_.p;
         a.tile_cols = has_nblist_ ? tile_cols_.p : nullptr;
         a.items = items_.p;
-        a.rows = rows_;
         a.M = M_;
         a.pair_idxs = pair_idxs_.p;
         a.scales = scales_.p;
         a.pair_sign = negated_ ? -1.0 : 1.0;
         a.g_dx = d_g_dx;
         a.g_dl = g_dl;
+        a.g_dl_at = d_g_dl;
         a.grad_p = d_grad_p;
         a.grad_w = d_grad_w;
         a.state = state_.p;
         int per_sm = 0;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_adjoint, ADJ_WARPS * 32, 0));
-        k_adjoint<<<std::max(1, per_sm) * num_sms(), ADJ_WARPS * 32, 0, stream>>>(a);
+        void (*kernel)(AdjointArgs) = rows_ == 32 ? k_adjoint<32> : rows_ == 16 ? k_adjoint<16> : k_adjoint<8>;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, ADJ_WARPS * 32, 0));
+        kernel<<<std::max(1, per_sm) * num_sms(), ADJ_WARPS * 32, 0, stream>>>(a);
         CK(cudaPeekAtLastError());
     }
 
@@ -1508,7 +1510,35 @@ tmnb_status tmnb_potential_adjoint_device(
     }
     return tmb::guarded([&] {
         as_nb(pot)->adjoint_device(
-            N, P, d_x, d_p, d_box, lambda, d_g_du_dx, g_du_dl, d_grad_p, d_grad_w, static_cast<cudaStream_t>(stream));
+            N, P, d_x, d_p, d_box, lambda, d_g_du_dx, g_du_dl, nullptr, d_grad_p, d_grad_w,
+            static_cast<cudaStream_t>(stream));
+    });
+}
+
+tmnb_status tmnb_potential_adjoint_device_all(
+    tmnb_potential *pot,
+    int N,
+    int P,
+    const double *d_x,
+    const double *d_p,
+    const double *d_box,
+    double lambda,
+    const double *d_g_du_dx,
+    const double *d_g_du_dl,
+    double *d_grad_p,
+    double *d_grad_w,
+    void *stream) {
+    if (tmnb_status s = check_handle(pot)) {
+        return s;
+    }
+    if (!d_g_du_dl) {
+        tmb::g_last_error = "upstream gradient of du_dl must be non-null";
+        return TMNB_ERR_INVALID_ARGUMENT;
+    }
+    return tmb::guarded([&] {
+        as_nb(pot)->adjoint_device(
+            N, P, d_x, d_p, d_box, lambda, d_g_du_dx, 0.0, d_g_du_dl, d_grad_p, d_grad_w,
+            static_cast<cudaStream_t>(stream));
     });
 }
 

@@ -371,8 +371,9 @@ class Potential:
 
     def adjoint_device(self, x, p, box, lam, g_du_dx, g_du_dl, grad_p, grad_w, stream=None):
         """Adds the vector-Jacobian product of (du_dx, du_dl) with upstream
-        (g_du_dx [N,3] float64, g_du_dl float) into grad_p [P] and grad_w [N]
-        (float64 device tensors): d/d params and d/d per-atom lambda offsets."""
+        (g_du_dx [N,3] float64, g_du_dl a float, or a float64 tensor of one
+        value on the device) into grad_p [P] and grad_w [N] (float64 device
+        tensors): d/d params and d/d per-atom lambda offsets."""
         import torch
 
         def addr(t):
@@ -384,10 +385,15 @@ class Potential:
             stream = torch.cuda.current_stream(x.device).cuda_stream
         elif hasattr(stream, "cuda_stream"):
             stream = stream.cuda_stream
+        on_device = (
+            isinstance(g_du_dl, torch.Tensor) and g_du_dl.device == x.device and g_du_dl.dtype == torch.float64
+            and g_du_dl.numel() == 1
+        )
+        call = self._lib.tmnb_potential_adjoint_device_all if on_device else self._lib.tmnb_potential_adjoint_device
         _lib.check(
-            self._lib.tmnb_potential_adjoint_device(
+            call(
                 self._h, x.shape[0], p.numel(), addr(x), addr(p), addr(box), float(lam), addr(g_du_dx),
-                float(g_du_dl), addr(grad_p), addr(grad_w), ctypes.c_void_p(stream),
+                addr(g_du_dl) if on_device else float(g_du_dl), addr(grad_p), addr(grad_w), ctypes.c_void_p(stream),
             )
         )
 

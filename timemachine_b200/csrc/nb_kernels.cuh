@@ -1697,10 +1697,10 @@ __device__ __forceinline__ void walk_item(
     const bool rows_alch = walk_load_rows(a, sm, lane, row_first, window);
     for (int t = 0; t < it.z; t++) {
         const unsigned j = a.tile_cols[((long long)it.y + t) * TILE + lane];
-        if (SKIP_DEP && __any_sync(FULL_MASK, j < (unsigned)a.S && a.lamdep[j])) {
-            continue;
+        if (!SKIP_DEP || !__any_sync(FULL_MASK, j < (unsigned)a.S && a.lamdep[j])) {
+            walk_tile<Real, U, DX, DL, DP, INTERP, RG>(a, sm, lane, row_first, rows_alch, j, window, b, out);
         }
-        walk_tile<Real, U, DX, DL, DP, INTERP, RG>(a, sm, lane, row_first, rows_alch, j, window, b, out);
+        // counted over all tiles, so that tiles left out do not put it off
         if ((t + 1) % sm.FLUSH_TILES == 0 && t + 1 < it.z) {
             walk_flush_rows(sm, lane, out, row_first, a.row_end);
         }

@@ -78,6 +78,8 @@ __device__ __forceinline__ SortArgs sort_args(const Rep &r) {
     sa.box = r.box;
     sa.set_atoms = nullptr;
     sa.n_first = r.N;
+    sa.offset = nullptr;
+    sa.first_atom = 0;
     sa.grid_bits = r.grid_bits;
     sa.hilbert = 1;
     sa.keys = r.keys;
@@ -147,7 +149,7 @@ __global__ void k_b_keys(const Rep *__restrict__ reps, const int2 *__restrict__ 
     if (!r.state->rebuild || r.state->error || k >= r.N) {
         return;
     }
-    bin_key(sort_args(r), k);
+    bin_key(sort_args(r), k, 0u);
 }
 
 __global__ void k_b_scan(const Rep *__restrict__ reps) {

@@ -732,24 +732,28 @@ __host__ __device__ __forceinline__ long long tile_base(const TileArgs &a, int g
 }
 
 constexpr int TB_WARPS = 8;
-// Column atoms the CTA holds before it sorts them into tiles; a full buffer is
-// sorted and its whole tiles are written. Groups of 16 rows list about 900
-// atoms at 100 atoms per nm^3.
+// Column atoms the CTA holds before it sorts them into tiles. Groups of 16
+// rows list about 900 atoms at 100 atoms per nm^3; a group that lists more
+// than fit is done again in rounds of TB_ROUND blocks, each followed by a
+// check, and a nearly full buffer is sorted and its whole tiles are written.
 constexpr int TB_COLS = 3072;
+constexpr int TB_ROUND = 32;
+constexpr int TB_WINDOWS = 16; // box tests per thread before the atoms are gone through
 // sort keys: lambda dependence x Lennard-Jones x 33 row counts
 constexpr int TB_KEYS = 2 * 2 * 33;
-// Tile-build CTAs per SM the compiler must fit (40 registers). The packed row
-// tests left to the compiler take 57 registers (4 CTAs/SM): measured on B200,
-// one rebuild 87.3 us with the scalar tests, 90.0 us packed at 57 registers,
-// 81.3 us packed at 40.
+// Tile-build CTAs per SM the compiler must fit (40 registers; 5 CTAs at 48
+// measured the same). The build is bound by instruction issue (ncu at 98,000
+// atoms: 75 % of issue slots), so what counts is what it does per column atom:
+// measured on B200, us of a forces call with a rebuild, testing every atom of a
+// passing block with three barriers per window of 256 blocks -> the atoms in
+// reach only, box tests of 16 windows at a time: 98,000 atoms 431 -> 397,
+// 22,840 137 -> 130. Loading the next block's atoms ahead: 434.
 #ifndef TMNB_TB_CTAS
 #define TMNB_TB_CTAS 6
 #endif
 
 struct TileBuildSmem {
-    float4 row_pos[TILE];
-    // the same positions as x, y, z arrays: element pair m holds rows 2m, 2m + 1
-    // (rows past the group's last lie out of every column's reach)
+    // row positions: element pair m holds rows 2m, 2m + 1 (NaN past the group's last)
     alignas(8) float row_x[TILE];
     alignas(8) float row_y[TILE];
     alignas(8) float row_z[TILE];
@@ -760,8 +764,8 @@ struct TileBuildSmem {
     unsigned char rem_keys[TILE];
     int bins[TB_KEYS]; // columns of each key, then the next position of each key
     int n_cols;
-    int cand[TB_WARPS * 32]; // column blocks of the current window that pass the box test
-    int warp_pass[TB_WARPS];
+    float4 queue[TB_WARPS][2 * TILE]; // column atoms in reach of the group's box: position, slot
+    unsigned passing[TB_WINDOWS * TB_WARPS]; // column blocks that pass the box test, one bit each
     int is_last;
 };
 
@@ -826,6 +830,58 @@ __device__ __forceinline__ int tb_emit(TileBuildSmem &sm, const TileArgs &a, int
     return n_out / TILE;
 }
 
+// Up to 32 column atoms (one per lane, `active`; slot in q.w) against the row
+// atoms: those within the list radius of one are collected with their key.
+__device__ __forceinline__ void tb_test_columns(
+    TileBuildSmem &sm, const TileArgs &a, const float4 q, const bool active, const bool shifted, const float r2, const float Lx, const float Ly, const float Lz, const float iLx, const float iLy, const float iLz) {
+    const int lane = threadIdx.x & 31;
+    const float rc2 = a.cutoff * a.cutoff;
+    float d2_min = 3.0e38f;
+    int near = 0; // row atoms within the cutoff
+    // two rows per packed FP32x2 test; a NaN row passes no comparison
+    const float2 qx = f2(q.x), qy = f2(q.y), qz = f2(q.z);
+    const float2 *rx2 = reinterpret_cast<const float2 *>(sm.row_x);
+    const float2 *ry2 = reinterpret_cast<const float2 *>(sm.row_y);
+    const float2 *rz2 = reinterpret_cast<const float2 *>(sm.row_z);
+    auto test = [&](const float2 dx, const float2 dy, const float2 dz) {
+        const float2 d2 = ffma2(dz, dz, ffma2(dy, dy, fmul2(dx, dx)));
+        d2_min = fminf(d2_min, fminf(d2.x, d2.y));
+        near += d2.x < rc2 ? 1 : 0;
+        near += d2.y < rc2 ? 1 : 0;
+    };
+    if (shifted) {
+        for (int r0 = 0; r0 < a.rows / 2; r0 += 4) {
+#pragma unroll
+            for (int r = r0; r < r0 + 4; r++) {
+                test(fsub2(rx2[r], qx), fsub2(ry2[r], qy), fsub2(rz2[r], qz));
+            }
+        }
+    } else {
+        const float2 lx = f2(-Lx), ly = f2(-Ly), lz = f2(-Lz), ix = f2(iLx), iy = f2(iLy), iz = f2(iLz);
+        for (int r = 0; r < a.rows / 2; r++) {
+            test(min_image2(fsub2(rx2[r], qx), lx, ix), min_image2(fsub2(ry2[r], qy), ly, iy),
+                 min_image2(fsub2(rz2[r], qz), lz, iz));
+        }
+    }
+    const bool hit = active && d2_min < r2;
+    const unsigned hmask = __ballot_sync(FULL_MASK, hit);
+    if (hmask == 0) {
+        return;
+    }
+    int at = 0;
+    if (lane == 0) {
+        at = atomicAdd(&sm.n_cols, __popc(hmask));
+    }
+    at = __shfl_sync(FULL_MASK, at, 0) + __popc(hmask & ((1u << lane) - 1));
+    if (hit && at < TB_COLS) {
+        const int s = __float_as_int(q.w);
+        const int key = (a.lamdep[s] ? 0 : 66) + (a.prm[s].z != 0.f ? 0 : 33) + 32 - near;
+        sm.cols[at] = (unsigned)s;
+        sm.keys[at] = (unsigned char)key;
+        atomicAdd(&sm.bins[key], 1);
+    }
+}
+
 __device__ __forceinline__ void build_tiles_cta(const TileArgs &a, const int rb, DevState *state) {
     __shared__ TileBuildSmem sm;
 
@@ -835,7 +891,6 @@ __device__ __forceinline__ void build_tiles_cta(const TileArgs &a, const int rb,
     const float Lx = (float)a.box[0], Ly = (float)a.box[4], Lz = (float)a.box[8];
     const float iLx = 1.0f / Lx, iLy = 1.0f / Ly, iLz = 1.0f / Lz;
     const float r2 = a.radius * a.radius;
-    const float rc2 = a.cutoff * a.cutoff;
     const float r2_box = (a.radius + 1e-4f) * (a.radius + 1e-4f);
     const int rows = a.rows;
     const int row_first = rb * rows;
@@ -883,8 +938,7 @@ __device__ __forceinline__ void build_tiles_cta(const TileArgs &a, const int rb,
         p.x = rc.x + wrap_delta(p.x - rc.x, Lx, iLx);
         p.y = rc.y + wrap_delta(p.y - rc.y, Ly, iLy);
         p.z = rc.z + wrap_delta(p.z - rc.z, Lz, iLz);
-        sm.row_pos[threadIdx.x] = p;
-        sm.row_x[threadIdx.x] = (int)threadIdx.x < row_n ? p.x : 1e18f;
+        sm.row_x[threadIdx.x] = (int)threadIdx.x < row_n ? p.x : __int_as_float(0x7fffffff);
         sm.row_y[threadIdx.x] = p.y;
         sm.row_z[threadIdx.x] = p.z;
     }
@@ -899,115 +953,105 @@ __device__ __forceinline__ void build_tiles_cta(const TileArgs &a, const int rb,
     const long long base_tile = tile_base(a, rb);
     const unsigned lane_lt = (1u << lane) - 1;
 
+    // The box tests (one column block per thread) leave a bit per block, then
+    // warp w goes through the set bits w, w + 8, w + 16 and w + 24 of every word:
+    // passing blocks cluster at nearby indices, so interleaving gives every warp
+    // about as many, without ranking them.
+    const int first_block = a.group ? a.cb_first : row_first / TILE;
     int tiles = 0;  // tiles written so far (uniform over the CTA)
     int n_have = 0; // columns collected (uniform over the CTA)
-    // Column blocks in windows of one block per thread: the box test of the
-    // window compacts the passing blocks in index order, then each warp takes
-    // an equal share of them. Passing blocks cluster at nearby indices, so a
-    // fixed split of the window by index would leave most warps idle.
-    for (int wbase = a.group ? a.cb_first : row_first / TILE; wbase < a.RB; wbase += TB_WARPS * 32) {
-        const int cb = wbase + (int)threadIdx.x;
-        bool pass = false;
-        if (cb < a.RB) {
-            const float4 cc = a.bb_ctr[cb];
-            const float4 ce = a.bb_ext[cb];
-            float dx = fmaxf(0.f, fabsf(wrap_delta(rc.x - cc.x, Lx, iLx)) - re.x - ce.x);
-            float dy = fmaxf(0.f, fabsf(wrap_delta(rc.y - cc.y, Ly, iLy)) - re.y - ce.y);
-            float dz = fmaxf(0.f, fabsf(wrap_delta(rc.z - cc.z, Lz, iLz)) - re.z - ce.z);
-            pass = dx * dx + dy * dy + dz * dz < r2;
-        }
-        const unsigned m = __ballot_sync(FULL_MASK, pass);
-        if (lane == 0) {
-            sm.warp_pass[warp] = __popc(m);
-        }
-        __syncthreads();
-        int base = 0, nc = 0;
-        for (int w = 0; w < TB_WARPS; w++) {
-            const int c = sm.warp_pass[w];
-            base += w < warp ? c : 0;
-            nc += c;
-        }
-        if (pass) {
-            sm.cand[base + __popc(m & lane_lt)] = cb;
-        }
-        __syncthreads();
-        for (int k0 = 0; k0 < nc;) {
-            if (TB_COLS - n_have < TB_WARPS * TILE) {
-                tiles += tb_emit(sm, a, n_have, base_tile + tiles, false);
-                n_have = n_have % TILE;
-            }
-            const int take = min(nc - k0, (TB_COLS - n_have) / TILE); // blocks whose atoms all fit
-            const int k_end = k0 + ((warp + 1) * take) / TB_WARPS;
-            for (int k = k0 + (warp * take) / TB_WARPS; k < k_end; k++) {
-                const int s = sm.cand[k] * TILE + lane;
-                const bool valid = s < S;
-                const float4 pj = valid ? a.posw[s] : make_float4(0.f, 0.f, 0.f, 0.f);
-                // an atom farther than the radius from the row block's box is
-                // farther than the radius from every row atom (widened test,
-                // conservative under rounding): skip its per-row test
-                const float wx = wrap_delta(pj.x - rc.x, Lx, iLx);
-                const float wy = wrap_delta(pj.y - rc.y, Ly, iLy);
-                const float wz = wrap_delta(pj.z - rc.z, Lz, iLz);
-                const float bx = fmaxf(0.f, fabsf(wx) - re.x);
-                const float by = fmaxf(0.f, fabsf(wy) - re.y);
-                const float bz = fmaxf(0.f, fabsf(wz) - re.z);
-                const bool need = valid && s >= col_lo && bx * bx + by * by + bz * bz < r2_box;
-                if (!__any_sync(FULL_MASK, need)) {
-                    continue;
+    for (bool rounds = false;; rounds = true) {
+        const int round = rounds ? TB_ROUND : TB_WINDOWS * TB_WARPS * TILE;
+        for (int c0 = first_block; c0 < a.RB; c0 += round) {
+            const int c_end = min(a.RB, c0 + round);
+            const int windows = (c_end - c0 + TB_WARPS * TILE - 1) / (TB_WARPS * TILE);
+            for (int i = 0; i < windows; i++) {
+                const int cb = c0 + i * TB_WARPS * TILE + (int)threadIdx.x;
+                bool pass = false;
+                if (cb < c_end) {
+                    const float4 cc = a.bb_ctr[cb];
+                    const float4 ce = a.bb_ext[cb];
+                    const float dx = fmaxf(0.f, fabsf(wrap_delta(rc.x - cc.x, Lx, iLx)) - re.x - ce.x);
+                    const float dy = fmaxf(0.f, fabsf(wrap_delta(rc.y - cc.y, Ly, iLy)) - re.y - ce.y);
+                    const float dz = fmaxf(0.f, fabsf(wrap_delta(rc.z - cc.z, Lz, iLz)) - re.z - ce.z);
+                    pass = dx * dx + dy * dy + dz * dz < r2;
                 }
-                float d2_min = 3.0e38f;
-                int near = 0; // row atoms within the cutoff
-                if (shifted) {
-                    // two rows per packed FP32x2 test
-                    const float2 qx = f2(rc.x + wx), qy = f2(rc.y + wy), qz = f2(rc.z + wz);
-                    const float2 *rx2 = reinterpret_cast<const float2 *>(sm.row_x);
-                    const float2 *ry2 = reinterpret_cast<const float2 *>(sm.row_y);
-                    const float2 *rz2 = reinterpret_cast<const float2 *>(sm.row_z);
-                    for (int r0 = 0; r0 < rows; r0 += 8) {
-#pragma unroll
-                        for (int r = r0; r < r0 + 8; r += 2) {
-                            const float2 dx = fsub2(rx2[r >> 1], qx);
-                            const float2 dy = fsub2(ry2[r >> 1], qy);
-                            const float2 dz = fsub2(rz2[r >> 1], qz);
-                            const float2 d2 = ffma2(dz, dz, ffma2(dy, dy, fmul2(dx, dx)));
-                            d2_min = fminf(d2_min, fminf(d2.x, d2.y));
-                            near += d2.x < rc2 ? 1 : 0;
-                            near += d2.y < rc2 ? 1 : 0;
-                        }
-                    }
-                } else {
-                    for (int r = 0; r < row_n; r++) {
-                        const float4 pi = sm.row_pos[r];
-                        const float dx = wrap_delta(pi.x - pj.x, Lx, iLx);
-                        const float dy = wrap_delta(pi.y - pj.y, Ly, iLy);
-                        const float dz = wrap_delta(pi.z - pj.z, Lz, iLz);
-                        const float d2 = dx * dx + dy * dy + dz * dz;
-                        d2_min = fminf(d2_min, d2);
-                        near += d2 < rc2 ? 1 : 0;
-                    }
-                }
-                const bool hit = need && d2_min < r2;
-                const unsigned hmask = __ballot_sync(FULL_MASK, hit);
-                if (hmask == 0) {
-                    continue;
-                }
-                int at = 0;
+                const unsigned m = __ballot_sync(FULL_MASK, pass);
                 if (lane == 0) {
-                    at = atomicAdd(&sm.n_cols, __popc(hmask));
-                }
-                at = __shfl_sync(FULL_MASK, at, 0) + __popc(hmask & lane_lt);
-                if (hit) {
-                    const int key = (a.lamdep[s] ? 0 : 66) + (a.prm[s].z != 0.f ? 0 : 33) + 32 - near;
-                    sm.cols[at] = (unsigned)s;
-                    sm.keys[at] = (unsigned char)key;
-                    atomicAdd(&sm.bins[key], 1);
+                    sm.passing[i * TB_WARPS + warp] = m;
                 }
             }
-            k0 += take;
+            __syncthreads();
+            int queued = 0; // atoms in the warp's queue
+            for (int b0 = 0; b0 < windows * TB_WARPS; b0 += TILE) {
+                const unsigned mine =
+                    b0 + lane < windows * TB_WARPS ? sm.passing[b0 + lane] & (0x01010101u << warp) : 0u;
+                unsigned words = __ballot_sync(FULL_MASK, mine != 0);
+                int word = 0;
+                for (unsigned m = 0; m != 0 || words != 0; m &= m - 1) {
+                    if (m == 0) {
+                        word = __ffs(words) - 1;
+                        words &= words - 1;
+                        m = __shfl_sync(FULL_MASK, mine, word);
+                    }
+                    const int s = (c0 + (b0 + word) * TILE + __ffs(m) - 1) * TILE + lane;
+                    const bool valid = s < S;
+                    const float4 pj = valid ? a.posw[s] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    // an atom farther than the radius from the row block's box is
+                    // farther than the radius from every row atom (widened test,
+                    // conservative under rounding): skip its per-row test
+                    const float wx = wrap_delta(pj.x - rc.x, Lx, iLx);
+                    const float wy = wrap_delta(pj.y - rc.y, Ly, iLy);
+                    const float wz = wrap_delta(pj.z - rc.z, Lz, iLz);
+                    const float bx = fmaxf(0.f, fabsf(wx) - re.x);
+                    const float by = fmaxf(0.f, fabsf(wy) - re.y);
+                    const float bz = fmaxf(0.f, fabsf(wz) - re.z);
+                    const bool need = valid && s >= col_lo && bx * bx + by * by + bz * bz < r2_box;
+                    // only the atoms in reach of the box (about half of a block)
+                    // go on to the row tests, 32 at a time
+                    const unsigned nmask = __ballot_sync(FULL_MASK, need);
+                    if (need) {
+                        sm.queue[warp][queued + __popc(nmask & lane_lt)] =
+                            make_float4(rc.x + wx, rc.y + wy, rc.z + wz, __int_as_float(s));
+                    }
+                    queued += __popc(nmask);
+                    if (queued >= TILE) {
+                        __syncwarp();
+                        tb_test_columns(sm, a, sm.queue[warp][lane], true, shifted, r2, Lx, Ly, Lz, iLx, iLy, iLz);
+                        queued -= TILE;
+                        const float4 rest = sm.queue[warp][TILE + lane];
+                        __syncwarp();
+                        sm.queue[warp][lane] = rest;
+                        __syncwarp();
+                    }
+                }
+            }
+            __syncwarp();
+            if (queued > 0) {
+                tb_test_columns(sm, a, sm.queue[warp][lane], lane < queued, shifted, r2, Lx, Ly, Lz, iLx, iLy, iLz);
+            }
             __syncthreads();
             n_have = sm.n_cols;
             __syncthreads(); // read by all before the next columns are added
+            if (!rounds && n_have > TB_COLS) {
+                break;
+            }
+            if (rounds && n_have + TB_ROUND * TILE > TB_COLS) {
+                tiles += tb_emit(sm, a, n_have, base_tile + tiles, false);
+                n_have = n_have % TILE;
+            }
         }
+        if (n_have <= TB_COLS) {
+            break;
+        }
+        // more columns than the buffer holds: again, in rounds
+        for (int k = threadIdx.x; k < TB_KEYS; k += TB_WARPS * 32) {
+            sm.bins[k] = 0;
+        }
+        if (threadIdx.x == 0) {
+            sm.n_cols = 0;
+        }
+        __syncthreads();
     }
     tiles += tb_emit(sm, a, n_have, base_tile + tiles, true);
     if (warp == 0) {

@@ -254,6 +254,27 @@ tmnb_status tmnb_potential_execute_batch_host(
     unsigned long long *h_du_dl,
     unsigned long long *h_u);
 
+/*
+ * tmnb_potential_execute_batch_host with the outputs decoded to FP64 as the
+ * reference's bindings decode them (timemachine/cpp/src/wrap_kernels.cpp:381-625),
+ * du_dl and u summed over the atoms. The decoding runs on the device.
+ */
+tmnb_status tmnb_potential_execute_decoded_host(
+    tmnb_potential *pot,
+    int coord_batches,
+    int N,
+    int param_batches,
+    int P,
+    int lambda_batches,
+    const double *h_x,       /* [coord_batches,N,3] */
+    const double *h_p,       /* [param_batches,P] */
+    const double *h_boxes,   /* [coord_batches,3,3] */
+    const double *h_lambdas, /* [lambda_batches] */
+    double *h_du_dx,         /* [E,N,3] or NULL, E = coord * param * lambda batches */
+    double *h_du_dp,         /* [E,P] or NULL */
+    double *h_du_dl,         /* [E] or NULL */
+    double *h_u);            /* [E] or NULL */
+
 /* Fixed-point du_dp to float with per-column exponents
  * (timemachine/cpp/src/nonbonded_all_pairs.cu:435-450). */
 tmnb_status tmnb_potential_du_dp_fixed_to_float(
@@ -560,6 +581,11 @@ tmnb_status tmnb_batch_evaluate(tmnb_batch *b, int compute_du_dx, int compute_du
 tmnb_status tmnb_batch_md(tmnb_batch *b, int n_steps, int chunk, int use_graph);
 
 tmnb_status tmnb_batch_synchronize(tmnb_batch *b);
+
+/* One replica's results of the last evaluation, decoded to FP64 on the device
+ * as tmnb_potential_execute_decoded_host decodes them (du_dl and u summed). */
+tmnb_status tmnb_batch_result(
+    tmnb_batch *b, int id, double *du_dx /* [N,3] */, double *du_dp /* [N,3] */, double *du_dl, double *u);
 
 /* Copies (synchronising) replica id's x [N,3] (which 0), v (1), box (2) as
  * doubles, or its outputs du_dx [N,3] (3), du_dp [N,3] (4), per-atom du_dl

@@ -42,6 +42,7 @@ SOURCES = [
     "pair_f64_r16_interp.cu",
 ]
 BUILD_DIR = os.path.join(HERE, "_build")
+MAX_WINDOWS = 32  # TMNB_MAX_WINDOWS: lambda windows of one multi-window call
 
 
 def build(verbose: bool = False, jobs: int = 0) -> str:
@@ -115,6 +116,8 @@ def _declare(lib):
     lib.tmnb_potential_execute_windows_device.argtypes = [vp, i, i, vp, vp, vp, i, vp, vp, vp, vp, vp, vp]
     lib.tmnb_potential_execute_windows_host.argtypes = [vp, i, i, vp, vp, vp, i, vp, vp, vp, vp, vp]
     lib.tmnb_potential_execute_batch_host.argtypes = [vp, i, i, i, i, i, vp, vp, vp, vp, vp, vp, vp, vp]
+    lib.tmnb_potential_execute_decoded_host.argtypes = [vp, i, i, i, i, i, vp, vp, vp, vp, vp, vp, vp, vp]
+    lib.tmnb_potential_execute_decoded_host.restype = ctypes.c_int
     lib.tmnb_potential_du_dp_fixed_to_float.argtypes = [vp, i, i, vp, vp]
     lib.tmnb_potential_set_nblist_padding.argtypes = [vp, d]
     lib.tmnb_potential_disable_hilbert_sort.argtypes = [vp]
@@ -172,6 +175,8 @@ def _declare(lib):
     lib.tmnb_batch_md.argtypes = [vp, i, i, i]
     lib.tmnb_batch_synchronize.argtypes = [vp]
     lib.tmnb_batch_get.argtypes = [vp, i, i, vp]
+    lib.tmnb_batch_result.argtypes = [vp, i, vp, vp, vp, vp]
+    lib.tmnb_batch_result.restype = ctypes.c_int
     lib.tmnb_batch_set.argtypes = [vp, i, i, vp]
     lib.tmnb_batch_error.argtypes = [vp, i, c_int_p]
     lib.tmnb_batch_stats.argtypes = [vp, i, c_int_p, c_int_p, c_int_p]

@@ -20,7 +20,6 @@ import time
 import numpy as np
 
 from . import _lib
-from .fixed_point import du_dp_fixed_to_float, fixed_to_float, sum_fixed
 from .md import langevin_coefficients
 
 _X, _V, _BOX, _DU_DX, _DU_DP, _DU_DL, _U = range(7)
@@ -160,7 +159,7 @@ class ReplicaBatch:
 
     # -- state -----------------------------------------------------------------
     def _get(self, rid, which, shape, dtype):
-        out = np.zeros(shape, dtype=dtype)
+        out = np.empty(shape, dtype=dtype)
         _lib.check(self._lib.tmnb_batch_get(self._h, int(rid), which, _p(out)))
         return out
 
@@ -198,8 +197,10 @@ class ReplicaBatch:
 
     def result(self, rid):
         """(du_dx, du_dp, du_dl, u) of the last evaluation, decoded as the reference decodes them."""
-        dx, dp, dl, u = self.result_fixed(rid)
-        return fixed_to_float(dx), du_dp_fixed_to_float(dp), fixed_to_float(sum_fixed(dl)), fixed_to_float(sum_fixed(u))
+        N = self._size(rid)
+        du_dx, du_dp, sums = np.empty((N, 3)), np.empty((N, 3)), np.empty(2)
+        _lib.check(self._lib.tmnb_batch_result(self._h, int(rid), _p(du_dx), _p(du_dp), _p(sums[:1]), _p(sums[1:])))
+        return du_dx, du_dp, float(sums[0]), float(sums[1])
 
     def error(self, rid):
         c = ctypes.c_int32()

@@ -18,6 +18,7 @@
 // owns one device arena; the descriptor table and block maps are rebuilt on
 // the host and uploaded, and captured graphs are discarded.
 #include "bonded_math.cuh"
+#include "decode.cuh"
 #include "engine.hpp"
 #include "md_math.cuh"
 #include "nb_kernels.cuh"
@@ -838,6 +839,38 @@ class BatchEngine {
         CK(cudaStreamSynchronize(stream_));
     }
 
+    // Replica `id`'s outputs of the last evaluation in FP64, du_dl and u summed.
+    void result(int id, double *du_dx, double *du_dp, double *du_dl, double *u) {
+        Slot &s = slot(id);
+        const Rep &r = s.rep;
+        const size_t n = 3 * (size_t)r.N;
+        DecodeArgs d;
+        d.K = 1;
+        d.du_dx = r.du_dx;
+        d.du_dp = r.du_dp;
+        d.n_dx = d.n_dp = n;
+        d.dp_columns = 1;
+        d.du_dl = r.du_dl;
+        d.u = r.u;
+        d.N = r.N;
+        d.error = nullptr;
+        const size_t head = decode_offset_dx(1);
+        if (decoded_.n < head + 2 * n) {
+            CK(cudaStreamSynchronize(stream_));
+            decoded_.alloc(head + 2 * n);
+        }
+        d.out = decoded_.p;
+        k_decode<<<decode_grid(d, num_sms()), DECODE_THREADS, 0, stream_>>>(d);
+        CK(cudaPeekAtLastError());
+        double sums[3];
+        CK(cudaMemcpyAsync(sums, d.out, sizeof(sums), cudaMemcpyDeviceToHost, stream_));
+        CK(cudaMemcpyAsync(du_dx, d.out + head, n * sizeof(double), cudaMemcpyDeviceToHost, stream_));
+        CK(cudaMemcpyAsync(du_dp, d.out + head + n, n * sizeof(double), cudaMemcpyDeviceToHost, stream_));
+        CK(cudaStreamSynchronize(stream_));
+        *du_dl = sums[1];
+        *u = sums[2];
+    }
+
     // Overwrites replica `id`'s coordinates (0), velocities (1) or box (2).
     void set(int id, int which, const double *in) {
         if (which < 0 || which > 2) {
@@ -1289,6 +1322,7 @@ class BatchEngine {
     DevBuf<Rep> table_;
     DevBuf<int2> ablk_, rbmap_, bmap_, amap_;
     DevBuf<int> prefix_, counter_, tprefix_, tcounter_;
+    DevBuf<double> decoded_; // one replica's decoded outputs (result())
     bpair_t pair_kernels_[3][16];
     int rows_ = 16; // slots per row group of every replica's tile list
     std::map<int, cudaGraphExec_t> graphs_;
@@ -1483,6 +1517,16 @@ tmnb_status tmnb_batch_get(tmnb_batch *b, int id, int which, void *out) {
         return null_argument();
     }
     return tmb::guarded([&] { b->impl->get(id, which, out); });
+}
+
+tmnb_status tmnb_batch_result(tmnb_batch *b, int id, double *du_dx, double *du_dp, double *du_dl, double *u) {
+    if (tmnb_status s = check_batch(b)) {
+        return s;
+    }
+    if (!du_dx || !du_dp || !du_dl || !u) {
+        return null_argument();
+    }
+    return tmb::guarded([&] { b->impl->result(id, du_dx, du_dp, du_dl, u); });
 }
 
 tmnb_status tmnb_batch_set(tmnb_batch *b, int id, int which, const double *in) {

@@ -10,6 +10,7 @@
 #include <stdexcept>
 #include <string>
 #include <utility>
+#include <vector>
 
 namespace tmb {
 
@@ -285,7 +286,19 @@ class PotentialBase {
         check_device_error(s);
     }
 
+    // execute_windows_host with the outputs decoded to FP64 on the device and
+    // du_dl / u summed there (nonbonded.cu). h_x / h_p: nullptr keeps the
+    // previous call's. Outputs: [K,N,3], [K,P], [K], [K], nullptr: not requested.
+    void execute_decoded_host(
+        int N, int P, const double *h_x, const double *h_p, const double *h_box, int K, const double *lambdas,
+        double *du_dx, double *du_dp, double *du_dl, double *u);
+
   protected:
+    // Device error word (nullptr: the potential has none), and whether du_dp
+    // has the nonbonded parameter columns' exponents.
+    virtual const int *device_error_word() const { return nullptr; }
+    virtual bool nonbonded_columns() const { return false; }
+
     void release_host_stream() {
         if (host_stream_) {
             cudaStreamDestroy(host_stream_);
@@ -294,6 +307,8 @@ class PotentialBase {
     }
     cudaStream_t host_stream_ = nullptr;
     DevBuf<double> hx_, hp_, hbox_;
+    DevBuf<double> hdec_; // decoded outputs
+    std::vector<double> hstage_;
     DevBuf<unsigned long long> hdx_, hdp_, hdl_, hu_;
 };
 

@@ -10,6 +10,7 @@
 //   Group     (timemachine/cpp/src/nonbonded_interaction_group.cu): pairs of
 //              one row atom and one column atom (the complement); slots hold
 //              the spatially sorted rows, then the sorted columns.
+#include "decode.cuh"
 #include "engine.hpp"
 #include "lambda_transform.hpp"
 #include "nb_adjoint.cuh"
@@ -960,6 +961,10 @@ class NonbondedPotential : public PotentialBase {
         (void)N;
     }
 
+  protected:
+    const int *device_error_word() const override { return &state_.p->error; }
+    bool nonbonded_columns() const override { return true; }
+
   private:
     Kind kind_;
     int N_;
@@ -1025,6 +1030,92 @@ class NonbondedPotential : public PotentialBase {
 } // namespace tmb
 
 namespace tmb {
+
+// What a small call waits for on the host is the number of copies and the
+// passes over the results, so the raw accumulators are one buffer (one clear),
+// a kernel decodes them, and outputs up to HOST_STAGE bytes come back in one
+// copy together with the error word; larger ones go straight to the caller's
+// arrays. Measured on B200 against four clears, five copies back and the
+// decoding in numpy: 900 atoms, all outputs 157 -> 84 us per call; 4 frames x 6
+// windows of 5,000 atoms 2,720 -> 1,054.
+constexpr size_t HOST_STAGE = 256 * 1024;
+
+void PotentialBase::execute_decoded_host(
+    int N, int P, const double *h_x, const double *h_p, const double *h_box, int K, const double *lambdas,
+    double *du_dx, double *du_dp, double *du_dl, double *u) {
+    if (!host_stream_) {
+        CK(cudaStreamCreateWithFlags(&host_stream_, cudaStreamNonBlocking));
+    }
+    cudaStream_t s = host_stream_;
+    const size_t nx = 3 * (size_t)N, np = (size_t)std::max(P, 0), kk = K;
+    hx_.ensure(nx);
+    hp_.ensure(std::max<size_t>(np, 1));
+    hbox_.ensure(9);
+    if (h_x) {
+        CK(cudaMemcpyAsync(hx_.p, h_x, nx * sizeof(double), cudaMemcpyHostToDevice, s));
+    }
+    if (h_p && np) {
+        CK(cudaMemcpyAsync(hp_.p, h_p, np * sizeof(double), cudaMemcpyHostToDevice, s));
+    }
+    CK(cudaMemcpyAsync(hbox_.p, h_box, 9 * sizeof(double), cudaMemcpyHostToDevice, s));
+    const size_t n_dx = du_dx ? kk * nx : 0, n_dp = du_dp ? kk * np : 0, n_dl = du_dl ? kk * N : 0, n_u = u ? kk * N : 0;
+    hdx_.ensure(n_dx + n_dp + n_dl + n_u);
+    unsigned long long *raw = hdx_.p;
+    if (n_dx + n_dp + n_dl + n_u > 0) {
+        CK(cudaMemsetAsync(raw, 0, (n_dx + n_dp + n_dl + n_u) * sizeof(*raw), s));
+    }
+    DecodeArgs d;
+    d.K = K;
+    d.du_dx = n_dx ? raw : nullptr;
+    d.du_dp = n_dp ? raw + n_dx : nullptr;
+    d.du_dl = n_dl ? raw + n_dx + n_dp : nullptr;
+    d.u = n_u ? raw + n_dx + n_dp + n_dl : nullptr;
+    d.n_dx = n_dx;
+    d.n_dp = n_dp;
+    d.dp_columns = nonbonded_columns() ? 1 : 0;
+    d.N = N;
+    d.error = device_error_word();
+    hdec_.ensure(decode_offset_dx(K) + n_dx + n_dp);
+    d.out = hdec_.p;
+    execute_windows_device(
+        N, P, hx_.p, hp_.p, hbox_.p, K, lambdas, const_cast<unsigned long long *>(d.du_dx),
+        const_cast<unsigned long long *>(d.du_dp), const_cast<unsigned long long *>(d.du_dl),
+        const_cast<unsigned long long *>(d.u), s);
+    k_decode<<<decode_grid(d, num_sms()), DECODE_THREADS, 0, s>>>(d);
+    CK(cudaPeekAtLastError());
+    const size_t head = decode_offset_dx(K), all = head + n_dx + n_dp;
+    const size_t staged = all * sizeof(double) <= HOST_STAGE ? all : head;
+    hstage_.resize(std::max(hstage_.size(), staged));
+    CK(cudaMemcpyAsync(hstage_.data(), d.out, staged * sizeof(double), cudaMemcpyDeviceToHost, s));
+    if (staged < all) {
+        if (n_dx) {
+            CK(cudaMemcpyAsync(du_dx, d.out + head, n_dx * sizeof(double), cudaMemcpyDeviceToHost, s));
+        }
+        if (n_dp) {
+            CK(cudaMemcpyAsync(du_dp, d.out + head + n_dx, n_dp * sizeof(double), cudaMemcpyDeviceToHost, s));
+        }
+    }
+    CK(cudaStreamSynchronize(s));
+    if (hstage_[0] != 0) {
+        check_device_error(s); // throws, and clears the word
+    }
+    if (staged == all) {
+        if (n_dx) {
+            memcpy(du_dx, hstage_.data() + head, n_dx * sizeof(double));
+        }
+        if (n_dp) {
+            memcpy(du_dp, hstage_.data() + head + n_dx, n_dp * sizeof(double));
+        }
+    }
+    for (int k = 0; k < K; k++) {
+        if (du_dl) {
+            du_dl[k] = hstage_[1 + k];
+        }
+        if (u) {
+            u[k] = hstage_[1 + K + k];
+        }
+    }
+}
 
 // FP32 FMA throughput probe: 8 independent FMA chains per thread, enough
 // resident warps to fill every SM; the denominator of the pair kernel's
@@ -1412,6 +1503,54 @@ tmnb_status tmnb_potential_execute_batch_host(
                         h_du_dp ? h_du_dp + e * P : nullptr,
                         h_du_dl ? h_du_dl + e * N : nullptr,
                         h_u ? h_u + e * N : nullptr);
+                    e += K;
+                }
+            }
+        }
+    });
+}
+
+tmnb_status tmnb_potential_execute_decoded_host(
+    tmnb_potential *pot,
+    int coord_batches,
+    int N,
+    int param_batches,
+    int P,
+    int lambda_batches,
+    const double *h_x,
+    const double *h_p,
+    const double *h_boxes,
+    const double *h_lambdas,
+    double *h_du_dx,
+    double *h_du_dp,
+    double *h_du_dl,
+    double *h_u) {
+    if (tmnb_status s = check_handle(pot)) {
+        return s;
+    }
+    if (coord_batches <= 0 || param_batches <= 0 || lambda_batches <= 0 || N <= 0 || P < 0 || !h_x || (P > 0 && !h_p) ||
+        !h_boxes || !h_lambdas) {
+        tmb::g_last_error = "invalid batch arguments";
+        return TMNB_ERR_INVALID_ARGUMENT;
+    }
+    return tmb::guarded([&] {
+        size_t e = 0;
+        for (int c = 0; c < coord_batches; c++) {
+            for (int p = 0; p < param_batches; p++) {
+                for (int l = 0; l < lambda_batches; l += tmb::MAX_WINDOWS) {
+                    const int K = std::min(tmb::MAX_WINDOWS, lambda_batches - l);
+                    pot->impl->execute_decoded_host(
+                        N,
+                        P,
+                        p == 0 && l == 0 ? h_x + (size_t)c * N * 3 : nullptr,
+                        l == 0 && (param_batches > 1 || c == 0) ? h_p + (size_t)p * P : nullptr,
+                        h_boxes + (size_t)c * 9,
+                        K,
+                        h_lambdas + l,
+                        h_du_dx ? h_du_dx + e * N * 3 : nullptr,
+                        h_du_dp ? h_du_dp + e * P : nullptr,
+                        h_du_dl ? h_du_dl + e : nullptr,
+                        h_u ? h_u + e : nullptr);
                     e += K;
                 }
             }

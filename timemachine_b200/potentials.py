@@ -18,7 +18,7 @@ import itertools
 import numpy as np
 
 from . import _lib
-from .fixed_point import FIXED_EXPONENT, fixed_to_float, sum_fixed
+from .fixed_point import FIXED_EXPONENT, sum_fixed
 
 __all__ = [
     "CustomOpWrapper",
@@ -128,7 +128,8 @@ class Potential:
         return self._lib.tmnb_potential_num_atoms(self._h)
 
     # -- host entry points ---------------------------------------------------
-    def _execute_fixed(self, coords, params, box, lam, du_dx, du_dp, du_dl, u):
+    @staticmethod
+    def _host_inputs(coords, params, box):
         coords = np.ascontiguousarray(coords, dtype=np.float64)
         params = np.ascontiguousarray(params, dtype=np.float64)
         box = np.ascontiguousarray(box, dtype=np.float64)
@@ -136,6 +137,25 @@ class Potential:
             raise RuntimeError("coords must have shape (N, 3)")
         if box.size != 9:
             raise RuntimeError("box must have shape (3, 3)")
+        return coords, params, box
+
+    def _execute_decoded(self, C, N, Pb, P, L, coords, params, boxes, lambdas, du_dx, du_dp, du_dl, u):
+        """Decoded outputs of the C * Pb * L evaluations (flat leading axis), None where not requested."""
+        E = C * Pb * L
+        out_dx = np.empty((E, N, 3)) if du_dx else None
+        out_dp = np.empty((E, P)) if du_dp else None
+        out_dl = np.empty(E) if du_dl else None
+        out_u = np.empty(E) if u else None
+        _lib.check(
+            self._lib.tmnb_potential_execute_decoded_host(
+                self._h, C, N, Pb, P, L, _ptr(coords), _ptr(params), _ptr(boxes), _ptr(lambdas), _ptr(out_dx),
+                _ptr(out_dp), _ptr(out_dl), _ptr(out_u),
+            )
+        )
+        return out_dx, out_dp, out_dl, out_u
+
+    def _execute_fixed(self, coords, params, box, lam, du_dx, du_dp, du_dl, u):
+        coords, params, box = self._host_inputs(coords, params, box)
         N = coords.shape[0]
         P = params.size
         out_dx = np.empty((N, 3), dtype=np.uint64) if du_dx else None
@@ -176,15 +196,18 @@ class Potential:
 
     def execute_selective(self, coords, params, box, lam, compute_du_dx, compute_du_dp, compute_du_dl, compute_u):
         """timemachine/cpp/src/wrap_kernels.cpp:552-625: tuple with None for outputs not requested."""
-        params = np.asarray(params, dtype=np.float64)
-        fdx, fdp, fdl, fu = self._execute_fixed(
-            coords, params, box, lam, compute_du_dx, compute_du_dp, compute_du_dl, compute_u
+        coords, params, box = self._host_inputs(coords, params, box)
+        lam = np.array([lam], dtype=np.float64)
+        N = coords.shape[0]
+        du_dx, du_dp, du_dl, u = self._execute_decoded(
+            1, N, 1, params.size, 1, coords, params, box, lam, compute_du_dx, compute_du_dp, compute_du_dl, compute_u
         )
-        du_dx = fixed_to_float(fdx) if compute_du_dx else None
-        du_dp = self._decode_dp(fdp).reshape(params.shape) if compute_du_dp else None
-        du_dl = fixed_to_float(sum_fixed(fdl)) if compute_du_dl else None
-        u = fixed_to_float(sum_fixed(fu)) if compute_u else None
-        return du_dx, du_dp, du_dl, u
+        return (
+            du_dx.reshape(N, 3) if compute_du_dx else None,
+            du_dp.reshape(params.shape) if compute_du_dp else None,
+            float(du_dl[0]) if compute_du_dl else None,
+            float(u[0]) if compute_u else None,
+        )
 
     def execute(self, coords, params, box, lam):
         """timemachine/cpp/src/wrap_kernels.cpp:339-380: (du_dx, du_dp, du_dl, u)."""
@@ -214,39 +237,15 @@ class Potential:
         Pb = params.shape[0]
         P = params.size // Pb
         L = lambdas.size
-        E = C * Pb * L
-        out_dx = np.empty((E, N, 3), dtype=np.uint64) if compute_du_dx else None
-        out_dp = np.empty((E, P), dtype=np.uint64) if compute_du_dp else None
-        out_dl = np.empty((E, N), dtype=np.uint64) if compute_du_dl else None
-        out_u = np.empty((E, N), dtype=np.uint64) if compute_u else None
-        _lib.check(
-            self._lib.tmnb_potential_execute_batch_host(
-                self._h,
-                C,
-                N,
-                Pb,
-                P,
-                L,
-                _ptr(coords),
-                _ptr(params),
-                _ptr(boxes),
-                _ptr(lambdas),
-                _ptr(out_dx),
-                _ptr(out_dp),
-                _ptr(out_dl),
-                _ptr(out_u),
-            )
+        out_dx, out_dp, out_dl, out_u = self._execute_decoded(
+            C, N, Pb, P, L, coords, params, boxes, lambdas, compute_du_dx, compute_du_dp, compute_du_dl, compute_u
         )
-        res = [None, None, None, None]
-        if compute_du_dx:
-            res[0] = fixed_to_float(out_dx).reshape(C, Pb, L, N, 3)
-        if compute_du_dp:
-            res[1] = self._decode_dp(out_dp).reshape((C, Pb, L) + params.shape[1:])
-        if compute_du_dl:
-            res[2] = np.array([fixed_to_float(sum_fixed(r)) for r in out_dl]).reshape(C, Pb, L)
-        if compute_u:
-            res[3] = np.array([fixed_to_float(sum_fixed(r)) for r in out_u]).reshape(C, Pb, L)
-        return tuple(res)
+        return (
+            out_dx.reshape(C, Pb, L, N, 3) if compute_du_dx else None,
+            out_dp.reshape((C, Pb, L) + params.shape[1:]) if compute_du_dp else None,
+            out_dl.reshape(C, Pb, L) if compute_du_dl else None,
+            out_u.reshape(C, Pb, L) if compute_u else None,
+        )
 
     def du_dp_fixed_to_float(self, N, P, du_dp):
         return self._decode_dp(np.asarray(du_dp, dtype=np.uint64).reshape(-1))
@@ -288,13 +287,16 @@ class Potential:
 
     def execute_windows(self, coords, params, box, lambdas):
         """(du_dx [K,N,3], du_dp [K,*params.shape], du_dl [K], u [K]) for K lambda windows."""
-        params = np.asarray(params, dtype=np.float64)
-        fdx, fdp, fdl, fu = self.execute_windows_fixed(coords, params, box, lambdas)
-        K = fdx.shape[0]
-        du_dp = self._decode_dp(fdp).reshape((K,) + params.shape)
-        du_dl = np.array([fixed_to_float(sum_fixed(r)) for r in fdl])
-        u = np.array([fixed_to_float(sum_fixed(r)) for r in fu])
-        return fixed_to_float(fdx), du_dp, du_dl, u
+        coords, params, box = self._host_inputs(coords, params, box)
+        lambdas = np.ascontiguousarray(np.atleast_1d(lambdas), dtype=np.float64)
+        N, K = coords.shape[0], lambdas.size
+        if K < 1 or K > _lib.MAX_WINDOWS:
+            # the error of the multi-window entry point
+            self.execute_windows_fixed(coords, params, box, lambdas)
+        du_dx, du_dp, du_dl, u = self._execute_decoded(
+            1, N, 1, params.size, K, coords, params, box, lambdas, True, True, True, True
+        )
+        return du_dx, du_dp.reshape((K,) + params.shape), du_dl, u
 
     # -- device entry point (torch tensors) -----------------------------------
     def execute_device(self, x, p, box, lam, du_dx=None, du_dp=None, du_dl=None, u=None, stream=None):

@@ -664,6 +664,7 @@ class BatchEngine {
     ~BatchEngine() {
         drop_graphs();
         reps_.clear();
+        decoded_.release(); // in the stream's order
         if (stream_) {
             cudaStreamDestroy(stream_);
         }
@@ -855,11 +856,15 @@ class BatchEngine {
         d.N = r.N;
         d.error = nullptr;
         const size_t head = decode_offset_dx(1);
-        if (decoded_.n < head + 2 * n) {
-            CK(cudaStreamSynchronize(stream_));
-            decoded_.alloc(head + 2 * n);
+        if (decoded_.n < (head + 2 * n) * sizeof(double)) {
+            // for the largest replica, so that reading them all allocates once
+            size_t most = n;
+            for (const auto &kv : reps_) {
+                most = std::max(most, 3 * (size_t)kv.second->rep.N);
+            }
+            decoded_.alloc((head + 2 * most) * sizeof(double), stream_);
         }
-        d.out = decoded_.p;
+        d.out = reinterpret_cast<double *>(decoded_.p);
         k_decode<<<decode_grid(d, num_sms()), DECODE_THREADS, 0, stream_>>>(d);
         CK(cudaPeekAtLastError());
         double sums[3];
@@ -1322,7 +1327,7 @@ class BatchEngine {
     DevBuf<Rep> table_;
     DevBuf<int2> ablk_, rbmap_, bmap_, amap_;
     DevBuf<int> prefix_, counter_, tprefix_, tcounter_;
-    DevBuf<double> decoded_; // one replica's decoded outputs (result())
+    StreamArena decoded_; // one replica's decoded outputs (result())
     bpair_t pair_kernels_[3][16];
     int rows_ = 16; // slots per row group of every replica's tile list
     std::map<int, cudaGraphExec_t> graphs_;

@@ -99,8 +99,8 @@ FLOPS_PER_PAIR = _table_sum("distance", "electrostatics", "forces", "charge deri
 FLOPS_PER_LJ_PAIR = _table_sum("lennard_jones (both atoms carry epsilon)")
 FLOPS_PER_ALCH_PAIR = _table_sum("lambda-dependent pair (an atom with a nonzero lambda offset)")
 # DRAM bytes (read + write) of one 12-window pair-kernel launch on this
-# workload, from an ncu capture of the same command (15.7 MB read, 0 written)
-PAIR_LAUNCH_DRAM_BYTES = 15.7e6
+# workload, from an ncu capture of the same command (13.4 MB read, 0 written)
+PAIR_LAUNCH_DRAM_BYTES = 13.4e6
 # stages of a call timed by tmnb_potential_last_stage_ms
 STAGE_PREPARE, STAGE_REBUILD, STAGE_PAIR, STAGE_FINALIZE = 0, 1, 2, 3
 
@@ -392,24 +392,24 @@ def hbm_roofline(N, K, ms, tiles, items, peak):
     prepare (k_check_prepare): reads x, the list's x, params (f64, 24 B each),
       plane + offset, slot order, lambda flag (13 B); writes K x 32 B of
       staged float4 coordinates + parameters and the flag.
-    rebuild (sort, scatter, block bounds, tile build; on a rebuild call):
-      reads x twice (keys, scatter) and params (LJ order); writes the slot
-      order, the list's x, the staging (K x 32 B), bounds; the tiles
-      (tiles x 32 column slots x 4 B) and work items (16 B).
-    finalize (k_finalize + accumulator reset): reads the 8 accumulator arrays
-      of the shared block and of the K window blocks (8 B each); adds K
-      windows of outputs (du_dx, du_dp 24 B, du_dl, u 8 B: read + write);
-      zeroes the blocks it read.
+    rebuild (slot order, staging, tile build; on a rebuild call): reads x
+      twice (keys, staging) and params (LJ order); writes the slot order, the
+      list's x, the staging (K x 32 B), bounds; the tiles (tiles x 32 column
+      slots x 4 B) and work items (16 B); zeroes the 8 accumulator arrays of
+      the shared block and of the K window blocks (8 B each).
+    finalize (k_finalize): reads those accumulators; adds K windows of outputs
+      (du_dx, du_dp 24 B, du_dl, u 8 B: read + write).
     """
     blocks = 1 + K if K > 1 else 1
     b_prepare = N * (24 + 24 + 24 + 13 + 1 + 32 * K)
     b_rebuild = N * (24 * 2 + 24 + 8 + 24 + 32 * K) + (N // 32 + 1) * 32 + tiles * 32 * 4 + items * 16
-    b_finalize = N * (8 * 8 * blocks * 2 + K * 64 * 2)
+    b_rebuild += N * 8 * 8 * blocks
+    b_finalize = N * (8 * 8 * blocks + K * 64 * 2)
     out = {}
     for name, b, t in [
         ("k_check_prepare", b_prepare, ms["prepare"]),
-        ("rebuild_chain (k_bin_keys..k_build_tiles)", b_rebuild, ms["rebuild"]),
-        ("k_finalize + reset", b_finalize, ms["finalize"]),
+        ("rebuild_chain (k_order_slots..k_build_tiles, accumulator reset)", b_rebuild, ms["rebuild"]),
+        ("k_finalize", b_finalize, ms["finalize"]),
     ]:
         gbs = b / (t * 1e-3) / 1e9
         out[name] = {"bytes": int(b), "ms": t, "achieved_gbs": gbs, "frac": gbs / peak}

@@ -324,7 +324,7 @@ tmnb_status tmnb_potential_copy_nblist(
 #define TMNB_STAGE_PREPARE 0  /* rebuild check, box checks, staging (k_check_prepare) */
 #define TMNB_STAGE_REBUILD 1  /* neighbour-list rebuild chain (returns at once when none is due) */
 #define TMNB_STAGE_PAIR 2     /* pair kernel */
-#define TMNB_STAGE_FINALIZE 3 /* scatter into the caller's outputs and accumulator reset */
+#define TMNB_STAGE_FINALIZE 3 /* scatter into the caller's outputs */
 tmnb_status tmnb_potential_enable_timing(tmnb_potential *pot, int on);
 tmnb_status tmnb_potential_last_stage_ms(tmnb_potential *pot, int stage, float *ms);
 tmnb_status tmnb_potential_last_pair_kernel_ms(tmnb_potential *pot, float *ms);

@@ -1197,15 +1197,14 @@ template <> struct Staged<double> {
 // Tile walk: the pairs of a tile (RG rows x 32 columns) that lie within the
 // cutoff, and only those.
 //
-// What bounds it: instruction issue, then the shared-memory pipe (ncu, forces
-// at 22,840 atoms: 71 % of issue slots, 28 of 32 lanes per instruction, shared
-// wavefronts half of the pipe's cycles; DRAM idle). The sweep of every row x
-// column that this replaced issued 69.8 M warp instructions there, the walk
-// 49.6 M. Kernel times on B200, before -> after, bit-identical: all outputs of
-// 12 windows at 22,840 atoms 157 -> 109 us (FP64 363 -> 239), forces of an MD
-// step 80.5 -> 68, all outputs at 98,000 atoms 480 -> 322; batch of 24 replicas
-// 1,568 -> 1,171 (all), 1,017 -> 795 (forces). 7 or 8 CTAs/SM instead of 6
-// change nothing; loading the next tile's columns ahead costs 2 to 6 %.
+// What bounds it: instruction issue and the shared-memory pipe (ncu, forces at
+// 22,840 atoms: 64 % of issue slots, 28.6 of 32 lanes per instruction, 65 % of
+// the L1 / shared wavefronts; DRAM idle). The sweep of every row x column that
+// this replaced issued 69.8 M warp instructions there, the walk 43.4 M. Kernel
+// times on B200 under ncu, before -> after, bit-identical: forces 92.3 -> 69.2 us,
+// all outputs of 12 windows 154 -> 104 (FP64 410 -> 209), batch of 64 replicas
+// 3.04 -> 2.56 ms. 7 or 8 CTAs/SM instead of 6 change nothing; loading the next
+// tile's columns ahead costs 2 to 6 %.
 //
 // Lane l owns column l of the tile: its atom and its sums stay in registers.
 // The tile's rows are staged in shared memory once per work item. A tile takes

@@ -163,3 +163,32 @@ def test_footprint_errors_and_autotune():
     want = _single_fixed(s, 0.0)
     got = b.result_fixed(rid)
     np.testing.assert_array_equal(got[0], want[0])
+
+
+def test_all_outputs_of_small_replicas_cost_little_more_than_forces():
+    """The all-outputs pair kernel runs at its arithmetic, not at the instruction
+    cache: an evaluation of 64 replicas of 1,500 atoms with every output took 1.4
+    times one of the forces alone before the tile walk, 2.1 times with a walk of
+    more code than the cache holds, and takes 1.3 times now."""
+    import torch
+
+    b = ReplicaBatch()
+    for k in range(64):
+        b.add(testsystems.system_of_size(1500, seed=3 + k % 4, n_ligand=37, min_edge=2.9), 0.4)
+    stream = torch.cuda.ExternalStream(b.stream)
+
+    def ms(**outputs):
+        best = np.inf
+        for _ in range(6):
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            start.record(stream)
+            for _ in range(5):
+                b.evaluate(**outputs)
+            end.record(stream)
+            end.synchronize()
+            best = min(best, start.elapsed_time(end) / 5)
+        return best
+
+    forces, everything = ms(du_dp=False, du_dl=False, u=False), ms()
+    print(f"forces {forces:.4f} ms, all outputs {everything:.4f} ms, ratio {everything / forces:.2f}")
+    assert everything < 1.7 * forces

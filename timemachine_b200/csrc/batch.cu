@@ -402,9 +402,20 @@ __device__ __forceinline__ PairArgs pair_args(const Rep &r) {
     return a;
 }
 
-// Persistent pair kernel over every replica's work units.
+// Persistent pair kernel over every replica's work units. What it needs of a
+// replica lies in registers, not in the launch's constants, and the warps of an
+// SM are in different walks (the replicas' boxes are small, so a tile's columns
+// often lie on both sides of the periodic boundary). With parameter derivatives
+// the three walks of a tile are 65 KB of code, spilled at 6 CTAs/SM, and the
+// warps wait for instructions (7.8 of 13 stall cycles per issue); so these
+// variants take the general image only (SHIFT off) and 5 CTAs/SM. Measured on
+// B200, us per launch, all outputs, three walks at 6 CTAs -> two at 5: 64
+// replicas of 1,500 atoms 447 -> 268 (the sweep of every slot: 353), 4 of 3,000
+// 98 -> 72, 16 of 6,000 465 -> 376, 24 of 14,000 1,372 -> 1,241, 4 of 22,840
+// 395 -> 354. Without derivatives (forces, energy) two walks are no faster (64 of
+// 1,500: 192 / 190 and 139 / 141; 4 of 22,840: 249 / 254 and 167 / 181).
 template <bool U, bool DX, bool DL, bool DP, int RG>
-__global__ void __launch_bounds__(128, (pair_min_ctas<float, U, DX, DL, DP, false, RG>()))
+__global__ void __launch_bounds__(128, DP ? 5 : (pair_min_ctas<float, U, DX, DL, DP, false, RG>()))
     k_b_pair(const Rep *__restrict__ reps, int R, const int *__restrict__ prefix, int *counter) {
     __shared__ WalkRows<float, DX, DP, false, RG> rows[4];
     WalkRows<float, DX, DP, false, RG> &sm = rows[threadIdx.x >> 5];
@@ -430,7 +441,7 @@ __global__ void __launch_bounds__(128, (pair_min_ctas<float, U, DX, DL, DP, fals
             }
             continue;
         }
-        walk_item<float, U, DX, DL, DP, false, false, RG>(a, sm, lane, r.items[local], 0, b, a.acc);
+        walk_item<float, U, DX, DL, DP, false, false, RG, !DP>(a, sm, lane, r.items[local], 0, b, a.acc);
     }
 }
 

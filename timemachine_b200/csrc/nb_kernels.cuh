@@ -1687,8 +1687,10 @@ __device__ __forceinline__ void walk_pairs(
 }
 
 // One tile: column j of the lane (>= S: none) against the staged rows; the
-// columns' sums go to their accumulators.
-template <typename Real, bool U, bool DX, bool DL, bool DP, bool INTERP, int RG>
+// columns' sums go to their accumulators. SHIFT: tiles whose columns have one
+// image each take a walk of their own (without it: less code, and the general
+// image for every tile).
+template <typename Real, bool U, bool DX, bool DL, bool DP, bool INTERP, int RG, bool SHIFT>
 __device__ __forceinline__ void walk_tile(
     const PairArgs &a,
     WalkRows<Real, DX, DP, INTERP, RG> &sm,
@@ -1716,14 +1718,18 @@ __device__ __forceinline__ void walk_tile(
     // coordinate give the same count, every row between them does, and the
     // column's image is one shift: -box * count (exact for counts up to 2) is
     // what the general form's fused multiply-add adds.
-    const Real nx = round_half_even(fmul(fsub(sm.lo[0], pwj.x), b.inv_x));
-    const Real ny = round_half_even(fmul(fsub(sm.lo[1], pwj.y), b.inv_y));
-    const Real nz = round_half_even(fmul(fsub(sm.lo[2], pwj.z), b.inv_z));
-    const bool one_image = nx == round_half_even(fmul(fsub(sm.hi[0], pwj.x), b.inv_x)) &&
-                           ny == round_half_even(fmul(fsub(sm.hi[1], pwj.y), b.inv_y)) &&
-                           nz == round_half_even(fmul(fsub(sm.hi[2], pwj.z), b.inv_z)) && fabs(nx) <= 2 &&
-                           fabs(ny) <= 2 && fabs(nz) <= 2;
-    const bool wrap = __any_sync(FULL_MASK, col_ok && !one_image);
+    Real nx = 0, ny = 0, nz = 0;
+    bool wrap = true;
+    if constexpr (SHIFT) {
+        nx = round_half_even(fmul(fsub(sm.lo[0], pwj.x), b.inv_x));
+        ny = round_half_even(fmul(fsub(sm.lo[1], pwj.y), b.inv_y));
+        nz = round_half_even(fmul(fsub(sm.lo[2], pwj.z), b.inv_z));
+        const bool one_image = nx == round_half_even(fmul(fsub(sm.hi[0], pwj.x), b.inv_x)) &&
+                               ny == round_half_even(fmul(fsub(sm.hi[1], pwj.y), b.inv_y)) &&
+                               nz == round_half_even(fmul(fsub(sm.hi[2], pwj.z), b.inv_z)) && fabs(nx) <= 2 &&
+                               fabs(ny) <= 2 && fabs(nz) <= 2;
+        wrap = __any_sync(FULL_MASK, col_ok && !one_image);
+    }
     // a column of the row group itself pairs with the rows before it
     const unsigned own = j - row_first;
     const unsigned valid = !col_ok ? 0u : (own < (unsigned)RG ? (1u << own) - 1 : FULL_MASK);
@@ -1735,7 +1741,7 @@ __device__ __forceinline__ void walk_tile(
         TMB_WALK(true, true);
     } else if (wrap) {
         TMB_WALK(false, true);
-    } else {
+    } else if constexpr (SHIFT) {
         TMB_WALK(false, false);
     }
 #undef TMB_WALK
@@ -1763,7 +1769,7 @@ __device__ __forceinline__ void walk_tile(
 
 // One work item: the tiles it.y .. it.y + it.z - 1 of row group it.x. With
 // skip_dep, tiles that hold a lambda-dependent atom are left out.
-template <typename Real, bool U, bool DX, bool DL, bool DP, bool INTERP, bool SKIP_DEP, int RG>
+template <typename Real, bool U, bool DX, bool DL, bool DP, bool INTERP, bool SKIP_DEP, int RG, bool SHIFT = true>
 __device__ __forceinline__ void walk_item(
     const PairArgs &a,
     WalkRows<Real, DX, DP, INTERP, RG> &sm,
@@ -1781,7 +1787,7 @@ __device__ __forceinline__ void walk_item(
     for (int t = 0; t < it.z; t++) {
         const unsigned j = a.tile_cols[((long long)it.y + t) * TILE + lane];
         if (!SKIP_DEP || !__any_sync(FULL_MASK, j < (unsigned)a.S && a.lamdep[j])) {
-            walk_tile<Real, U, DX, DL, DP, INTERP, RG>(a, sm, lane, row_first, rows_alch, j, window, b, out);
+            walk_tile<Real, U, DX, DL, DP, INTERP, RG, SHIFT>(a, sm, lane, row_first, rows_alch, j, window, b, out);
         }
         // counted over all tiles, so that tiles left out do not put it off
         if ((t + 1) % sm.FLUSH_TILES == 0 && t + 1 < it.z) {

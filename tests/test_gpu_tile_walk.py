@@ -12,6 +12,7 @@ from scipy.spatial import cKDTree
 
 from tests.helpers import f32_round, random_params
 from timemachine_b200 import potentials as P
+from timemachine_b200 import testsystems
 
 pytestmark = pytest.mark.gpu
 
@@ -118,3 +119,49 @@ def test_rebuild_paths(n):
     _assert_same([multi[k][0] if k < 2 else multi[k][0].sum(dtype=np.uint64) for k in range(4)], want)
     energy = _fixed(impl, x, p, box, 0.3, (False, False, False, True))
     _assert_same(energy, want)
+
+
+@pytest.mark.parametrize("n", [6000, 33000])  # the sort in one cluster, and as three kernels
+def test_only_compact_sites_take_the_first_slots(n):
+    """Atoms with a lambda offset sit in the first slots where they lie together;
+    where they lie in two places or anywhere, row groups that held several of them
+    would list the columns around all (of two places 1.3 times, of many over twice
+    the widest list without the rule), so after the first rebuild they keep the
+    plain order. The sums are the pair list's either way."""
+    s = testsystems.system_of_size(n, seed=n, n_ligand=40)
+    x, p, N = f32_round(s.x), f32_round(s.params), s.N
+    far = np.argsort((np.minimum(s.x, np.diag(s.box) - s.x) ** 2).sum(axis=1))[:24]  # a corner of the box
+    layouts = {
+        "none": [],
+        "ligand": s.ligand_idxs,
+        "two": np.concatenate([s.ligand_idxs, far]),
+        "anywhere": np.random.default_rng(n).choice(N, N // 100, replace=False),
+    }
+    plane, widest = np.zeros(N, np.int32), {}
+    for name, idxs in layouts.items():
+        offset = np.zeros(N, np.int32)
+        offset[idxs] = 1
+        impl = P.NonbondedAllPairs(plane, offset, s.beta, s.cutoff).unbound_impl(np.float32)
+        plain = P.NonbondedAllPairs(plane, offset, s.beta, s.cutoff).unbound_impl(np.float32)
+        plain.disable_hilbert_sort()
+        for shift in (0.0, 0.3, 0.0):
+            _assert_same(_fixed(impl, f32_round(x + shift), p, s.box, 0.3), _fixed(plain, f32_round(x + shift), p, s.box, 0.3))
+        perm, tiles, _ = impl.get_nblist()
+        assert np.array_equal(np.sort(perm), np.arange(N))
+        widest[name] = max(len(t) for t in tiles)
+        together = set(perm[: len(idxs) // 16 * 16]) <= set(idxs)  # full row groups
+        assert together == (name in ("none", "ligand"))
+    print(widest)
+    for name in ("ligand", "two", "anywhere"):
+        assert widest[name] <= 1.2 * widest["none"]
+    # many windows and many such atoms: first wherever they are
+    offset = np.zeros(N, np.int32)
+    offset[np.random.default_rng(n).choice(N, N // 30, replace=False)] = 1
+    impl = P.NonbondedAllPairs(plane, offset, s.beta, s.cutoff).unbound_impl(np.float32)
+    for shift in (0.0, 0.3):
+        multi = impl.execute_windows_fixed(f32_round(x + shift), p, s.box, np.array([0.3, 0.9]))
+        assert set(impl.get_nblist()[0][: N // 30 // 16 * 16]) <= set(np.flatnonzero(offset))
+    plain = P.NonbondedAllPairs(plane, offset, s.beta, s.cutoff).unbound_impl(np.float32)
+    plain.disable_hilbert_sort()
+    _assert_same([multi[k][0] if k < 2 else multi[k][0].sum(dtype=np.uint64) for k in range(4)],
+                 _fixed(plain, f32_round(x + 0.3), p, s.box, 0.3))

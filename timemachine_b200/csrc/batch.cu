@@ -80,7 +80,9 @@ __device__ __forceinline__ SortArgs sort_args(const Rep &r) {
     sa.set_atoms = nullptr;
     sa.n_first = r.N;
     sa.offset = nullptr;
-    sa.first_atom = 0;
+    sa.site_atoms = nullptr;
+    sa.n_site = 0;
+    sa.site_always = false;
     sa.grid_bits = r.grid_bits;
     sa.hilbert = 1;
     sa.keys = r.keys;
@@ -150,7 +152,7 @@ __global__ void k_b_keys(const Rep *__restrict__ reps, const int2 *__restrict__ 
     if (!r.state->rebuild || r.state->error || k >= r.N) {
         return;
     }
-    bin_key(sort_args(r), k, 0u);
+    bin_key(sort_args(r), k, false, 0u);
 }
 
 __global__ void k_b_scan(const Rep *__restrict__ reps) {
@@ -322,6 +324,7 @@ __global__ void __launch_bounds__(TB_WARPS * 32, TMNB_TB_CTAS)
         ta.cb_first = 0;
         ta.radius = (float)(r.cutoff + r.padding + 1e-5);
         ta.cutoff = (float)r.cutoff;
+        ta.n_site = 0;
         ta.box = r.box;
         ta.posw = r.posw;
         ta.prm = r.prm;

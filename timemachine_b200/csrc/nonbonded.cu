@@ -172,17 +172,16 @@ class NonbondedPotential : public PotentialBase {
             // which multi-window calls evaluate once per window, instead of those
             // atoms' cells and the cells around them (12 windows at 22,840 atoms
             // with a 40-atom ligand 125.4 -> 113.4 us per call on B200, FP64 252 ->
-            // 225; 2,500 atoms 46.5 -> 37.0). Many such atoms would make every row
-            // group wider, so above one in 16 they keep the plain order.
+            // 225; 2,500 atoms 46.5 -> 37.0). Above one in 16 they keep the plain order.
             std::vector<int> with_offset;
             for (int s = 0; s < S_; s++) {
                 if (h_offset_[perm[s]] != 0) {
                     with_offset.push_back((int)perm[s]);
                 }
             }
-            const int n_offset = (int)with_offset.size();
-            first_dep_ = n_offset > 0 ? with_offset[n_offset / 2] : 0;
-            dep_first_ = kind != Kind::Group && n_offset > 0 && n_offset <= S_ / 16;
+            if (kind != Kind::Group && with_offset.size() <= (size_t)S_ / 16) {
+                site_atoms_.upload(with_offset.data(), with_offset.size());
+            }
             RB_ = (S_ + TILE - 1) / TILE;
             cb_first_ = kind == Kind::Group ? NR_ / TILE : 0;
             nb_x_.alloc(3 * (size_t)N);
@@ -193,7 +192,7 @@ class NonbondedPotential : public PotentialBase {
             int b = (int)std::ceil(std::log2(std::cbrt(std::max(1.0, S_ / 8.0))));
             grid_bits_ = std::min(6, std::max(2, b));
             keys_.alloc(S_);
-            const size_t bins = ((size_t)1 << (3 * grid_bits_)) * (kind == Kind::Group ? 2 : 1) + (dep_first_ ? FIRST_BINS : 0);
+            const size_t bins = ((size_t)1 << (3 * grid_bits_)) * (kind == Kind::Group ? 2 : 1);
             bin_count_.alloc(bins);
             bin_count_.zero();
             bin_cursor_.alloc(bins);
@@ -711,8 +710,14 @@ class NonbondedPotential : public PotentialBase {
         sa.box = d_box;
         sa.set_atoms = set_atoms_.p;
         sa.n_first = kind_ == Kind::Group ? NR_ : S_;
-        sa.offset = dep_first_ ? offset_.p : nullptr;
-        sa.first_atom = first_dep_;
+        sa.offset = site_atoms_.n > 0 ? offset_.p : nullptr;
+        sa.site_atoms = site_atoms_.p;
+        sa.n_site = (int)site_atoms_.n;
+        // Many such atoms are worth the first slots to a multi-window call also where
+        // their row groups are wide: 12 windows with a rebuild, plain order / first
+        // slots, 8,000 / 22,840 / 98,000 atoms: 1 % of the atoms, anywhere in the box,
+        // 167 / 172, 391 / 366, 1,509 / 1,736 us; 3 % 252 / 193, 640 / 430, 2,505 / 2,128.
+        sa.site_always = K > 1 && site_atoms_.n * 64 > (size_t)S_;
         sa.grid_bits = grid_bits_;
         sa.hilbert = hilbert_ ? 1 : 0;
         sa.keys = keys_.p;
@@ -729,6 +734,7 @@ class NonbondedPotential : public PotentialBase {
         ta.cb_first = cb_first_;
         ta.radius = (float)(cutoff_ + padding_ + 1e-5);
         ta.cutoff = (float)cutoff_;
+        ta.n_site = (int)site_atoms_.n;
         ta.box = d_box;
         ta.posw = posw_.p;
         ta.prm = prm_.p;
@@ -985,8 +991,7 @@ class NonbondedPotential : public PotentialBase {
     int n_row_blocks_ = 0; // blocks whose slots act as rows
     int cb_first_ = 0;     // interaction group: first column block
     int grid_bits_ = 4;
-    bool dep_first_ = false; // atoms with a lambda offset sort first
-    int first_dep_ = 0;      // one of them
+    DevBuf<int> site_atoms_; // atoms with a lambda offset that may take the first slots
     int chunk_ = 1; // item capacity: one item per tile at most
     std::vector<std::pair<pair_kernel_t, int>> grid_cache_;
     // slots per row group of the tile list; 16 measured fastest on B200 at

@@ -4,8 +4,10 @@ staged copy and for larger ones, every output selection, and after an error."""
 
 import numpy as np
 import pytest
+import torch
 
 from tests.helpers import f32_round
+from timemachine_b200 import _lib
 from timemachine_b200 import potentials as P
 from timemachine_b200 import testsystems
 from timemachine_b200.batch import ReplicaBatch
@@ -71,3 +73,22 @@ def test_replica_results():
         dx, dp, dl, u = b.result_fixed(rid)
         want = fixed_to_float(dx), du_dp_fixed_to_float(dp), fixed_to_float(sum_fixed(dl)), fixed_to_float(sum_fixed(u))
         _same(b.result(rid), want)
+
+
+def test_replica_results_after_a_change_of_priority():
+    """The workspace of the results outlives the stream it was allocated on: it
+    grows and is freed on the batch's current one."""
+    b = ReplicaBatch()
+    ids = []
+    for n, priority in ((300, -1), (2600, 0), (5000, None)):  # each larger: the workspace grows
+        s = testsystems.system_of_size(n, seed=n, n_ligand=10, min_edge=2.9)
+        ids.append(b.add(s, 0.4))
+        b.evaluate()
+        for rid in ids:
+            dx, dp, dl, u = b.result_fixed(rid)
+            want = fixed_to_float(dx), du_dp_fixed_to_float(dp), fixed_to_float(sum_fixed(dl)), fixed_to_float(sum_fixed(u))
+            _same(b.result(rid), want)
+        if priority is not None:
+            _lib.check(b._lib.tmnb_batch_set_priority(b._h, priority))
+    del b
+    torch.cuda.synchronize()  # raises what the frees may have left

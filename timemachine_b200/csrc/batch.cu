@@ -955,6 +955,7 @@ class BatchEngine {
         for (auto &kv : reps_) {
             kv.second->arena.stream = s;
         }
+        decoded_.stream = s;
         CK(cudaStreamDestroy(stream_));
         stream_ = s;
     }

@@ -13,6 +13,7 @@ from scipy.spatial import cKDTree
 from tests.helpers import f32_round, random_params
 from timemachine_b200 import potentials as P
 from timemachine_b200 import testsystems
+from timemachine_b200.fixed_point import fixed_to_float
 
 pytestmark = pytest.mark.gpu
 
@@ -165,3 +166,30 @@ def test_only_compact_sites_take_the_first_slots(n):
     plain.disable_hilbert_sort()
     _assert_same([multi[k][0] if k < 2 else multi[k][0].sum(dtype=np.uint64) for k in range(4)],
                  _fixed(plain, f32_round(x + 0.3), p, s.box, 0.3))
+
+
+@pytest.mark.parametrize("n", [200, 3000, 9000])
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_an_atom_without_a_position_pairs_with_none(n, value):
+    """One coordinate of an atom is not a number; the others keep all their pairs,
+    also those that share its row group and its block. The atom is alone in having
+    a lambda offset, so it is the first of its group."""
+    s = testsystems.system_of_size(n, seed=n, n_ligand=5, min_edge=2.9)
+    x, p, N = f32_round(s.x), f32_round(s.params), s.N
+    plane, offset = np.zeros(N, np.int32), np.zeros(N, np.int32)
+    lost = int(s.ligand_idxs[2])
+    offset[lost] = 1
+    rest = np.arange(N) != lost
+    ref = P.NonbondedAllPairs(plane[rest], offset[rest], s.beta, s.cutoff).unbound_impl(np.float32)
+    want = _fixed(ref, x[rest], p[rest], s.box, 0.0)
+    for axis in range(3):
+        y = x.copy()
+        y[lost, axis] = value
+        for precision in (np.float32, np.float64):
+            impl = P.NonbondedAllPairs(plane, offset, s.beta, s.cutoff).unbound_impl(precision)
+            dx, dp, dl, u = _fixed(impl, y, p, s.box, 0.0)
+            assert not dx[lost].any() and not dp.reshape(N, 3)[lost].any()
+            if precision == np.float32:
+                _assert_same((dx[rest], dp.reshape(N, 3)[rest].reshape(-1), dl, u), want)
+            else:
+                np.testing.assert_allclose(fixed_to_float(u), fixed_to_float(want[3]), rtol=1e-5)

@@ -529,6 +529,10 @@ static __global__ void k_bin_scatter(SortArgs sa, unsigned *perm, const DevState
 
 __device__ __forceinline__ float wrap_delta(float d, float L, float inv_L) { return d - L * rintf(d * inv_L); }
 
+// What the atoms of a block are imaged next to: its first atom's coordinate (any
+// other where that one is infinite or NaN, else the whole block would be lost with it).
+__device__ __forceinline__ float box_reference(float first) { return fabsf(first) < 3.0e38f ? first : 0.f; }
+
 // Bounding box of the 32-slot block rb (one warp) from its atoms' positions p.
 __device__ __forceinline__ void block_bounds_warp(
     const bool valid, const float4 p, const double *box, int rb, float4 *bb_ctr, float4 *bb_ext) {
@@ -536,9 +540,9 @@ __device__ __forceinline__ void block_bounds_warp(
     const float Lx = (float)box[0], Ly = (float)box[4], Lz = (float)box[8];
     const float iLx = 1.0f / Lx, iLy = 1.0f / Ly, iLz = 1.0f / Lz;
     {
-        const float rx = __shfl_sync(FULL_MASK, p.x, 0);
-        const float ry = __shfl_sync(FULL_MASK, p.y, 0);
-        const float rz = __shfl_sync(FULL_MASK, p.z, 0);
+        const float rx = box_reference(__shfl_sync(FULL_MASK, p.x, 0));
+        const float ry = box_reference(__shfl_sync(FULL_MASK, p.y, 0));
+        const float rz = box_reference(__shfl_sync(FULL_MASK, p.z, 0));
         float dx = wrap_delta(p.x - rx, Lx, iLx);
         float dy = wrap_delta(p.y - ry, Ly, iLy);
         float dz = wrap_delta(p.z - rz, Lz, iLz);
@@ -943,9 +947,9 @@ __device__ __forceinline__ void build_tiles_cta(const TileArgs &a, const int rb,
         // the row group's box, as block_bounds_warp computes a 32-slot block's
         const bool valid = lane < row_n;
         const float4 p = valid ? a.posw[row_first + lane] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float rx = __shfl_sync(FULL_MASK, p.x, 0);
-        const float ry = __shfl_sync(FULL_MASK, p.y, 0);
-        const float rz = __shfl_sync(FULL_MASK, p.z, 0);
+        const float rx = box_reference(__shfl_sync(FULL_MASK, p.x, 0));
+        const float ry = box_reference(__shfl_sync(FULL_MASK, p.y, 0));
+        const float rz = box_reference(__shfl_sync(FULL_MASK, p.z, 0));
         const float dx = wrap_delta(p.x - rx, Lx, iLx);
         const float dy = wrap_delta(p.y - ry, Ly, iLy);
         const float dz = wrap_delta(p.z - rz, Lz, iLz);

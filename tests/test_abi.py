@@ -159,3 +159,17 @@ def test_create_without_gpu_fails_loudly():
 def test_bound_impl_requires_params():
     with pytest.raises(ValueError, match="not been bound"):
         P.NonbondedAllPairs([0], [0], 2.0, 1.1).bound_impl(np.float32)
+
+
+@pytest.mark.parametrize("lam", [None, [0.1, 0.2], np.array([0.1, 0.2]), 1j])
+def test_host_calls_refuse_a_lambda_that_is_not_one_number(monkeypatch, lam):
+    impl = P.Potential.__new__(P.Potential)
+    impl._h, impl._lib = None, None
+    monkeypatch.setattr(P.Potential, "_execute_decoded", lambda *a: (np.zeros((1, 2, 3)),) + 3 * (None,))
+    x, p, box = np.zeros((2, 3)), np.zeros((2, 3)), np.eye(3)
+    for value in (0.5, 1, np.float32(0.25), np.array(0.5)):
+        impl.execute_du_dx(x, p, box, value)
+    with pytest.raises(TypeError):
+        impl.execute_du_dx(x, p, box, lam)
+    with pytest.raises(TypeError):
+        impl.execute_selective(x, p, box, lam, True, False, False, False)

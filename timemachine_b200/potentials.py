@@ -197,7 +197,7 @@ class Potential:
     def execute_selective(self, coords, params, box, lam, compute_du_dx, compute_du_dp, compute_du_dl, compute_u):
         """timemachine/cpp/src/wrap_kernels.cpp:552-625: tuple with None for outputs not requested."""
         coords, params, box = self._host_inputs(coords, params, box)
-        lam = np.array([lam], dtype=np.float64)
+        lam = np.array([float(lam)])  # one number: None or several are refused
         N = coords.shape[0]
         du_dx, du_dp, du_dl, u = self._execute_decoded(
             1, N, 1, params.size, 1, coords, params, box, lam, compute_du_dx, compute_du_dp, compute_du_dl, compute_u

@@ -40,3 +40,35 @@ def test_walk_against_oracle(n, rows):
     for gp, gw in got:
         for ref, val in ((rp, gp), (rw, gw)):
             assert np.max(np.abs(ref - val)) <= 1e-10 * max(1.0, np.max(np.abs(ref)))
+
+
+def test_upstream_value_still_being_computed_while_another_stream_is_named():
+    """The upstream gradient of du_dl is taken in the order of the stream that
+    computes it, and its memory may go to another tensor after the call."""
+    n = 600
+    c = small_water_case(np.random.default_rng(n), n, planes=(-1, 2), offsets=(-1, 2))
+    impl = P.Nonbonded(c["exclusion_idxs"], c["scales"], c["plane"], c["offset"], 2.0, 1.2).unbound_impl(np.float32)
+    x, p, box = to_dev(f32_round(c["x"])), to_dev(f32_round(c["params"])).reshape(-1), to_dev(c["box"])
+    G = torch.zeros((n, 3), dtype=torch.float64, device="cuda")
+    side = torch.cuda.Stream()
+
+    def vjp(g, **kw):
+        gp, gw = torch.zeros(3 * n, dtype=torch.float64, device="cuda"), torch.zeros(n, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        g = g()
+        impl.adjoint_device(x, p, box, 0.4, G, g, gp, gw, **kw)
+        del g
+        torch.full((1,), 5.0, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        return gp.cpu().numpy(), gw.cpu().numpy()
+
+    def late():  # 0.7, some milliseconds from now
+        g = torch.zeros(1, dtype=torch.float64, device="cuda")
+        torch.cuda._sleep(20_000_000)
+        return g.add_(0.7)
+
+    want = vjp(lambda: 0.7)
+    assert np.abs(want[1]).max() > 0
+    for kw in ({}, {"stream": side}, {"stream": side.cuda_stream}):
+        for a, b in zip(vjp(late, **kw), want):
+            np.testing.assert_allclose(a, b, rtol=0, atol=1e-10 * max(1.0, np.abs(b).max()))

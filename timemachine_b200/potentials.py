@@ -374,7 +374,7 @@ class Potential:
     def adjoint_device(self, x, p, box, lam, g_du_dx, g_du_dl, grad_p, grad_w, stream=None):
         """Adds the vector-Jacobian product of (du_dx, du_dl) with upstream
         (g_du_dx [N,3] float64, g_du_dl a float, or a float64 tensor of one
-        value on the device) into grad_p [P] and grad_w [N] (float64 device
+        value on the device, waited for when `stream` is given) into grad_p [P] and grad_w [N] (float64 device
         tensors): d/d params and d/d per-atom lambda offsets."""
         import torch
 
@@ -383,14 +383,17 @@ class Potential:
                 raise RuntimeError("device tensors must be contiguous")
             return ctypes.c_void_p(t.data_ptr())
 
+        # read by the kernel on the stream that the value was computed on; on a stream
+        # that the caller names it could run before that one, or after the value's memory
+        # has gone to another tensor
+        on_device = (
+            stream is None and isinstance(g_du_dl, torch.Tensor) and g_du_dl.device == x.device and g_du_dl.dtype == torch.float64
+            and g_du_dl.numel() == 1
+        )
         if stream is None:
             stream = torch.cuda.current_stream(x.device).cuda_stream
         elif hasattr(stream, "cuda_stream"):
             stream = stream.cuda_stream
-        on_device = (
-            isinstance(g_du_dl, torch.Tensor) and g_du_dl.device == x.device and g_du_dl.dtype == torch.float64
-            and g_du_dl.numel() == 1
-        )
         call = self._lib.tmnb_potential_adjoint_device_all if on_device else self._lib.tmnb_potential_adjoint_device
         _lib.check(
             call(

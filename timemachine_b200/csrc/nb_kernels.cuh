@@ -1277,11 +1277,17 @@ template <> struct Staged<double> {
 // A row's sums are met by several lanes in a step and live in shared memory as
 // two 32-bit limbs (bits 0-23 and 24-55 of the fixed-point value): 32-bit
 // shared-memory additions are native, 64-bit ones are compare-and-swap loops.
-// 64 additions of values below 2^49 fit the limbs exactly; larger values (and
+// LIMB_ADDITIONS values up to LIMB_MAX fit the limbs exactly; larger ones (and
 // NaN) go to the row's global accumulator as a whole. Lane l starts its walk at
 // row l mod RG and each RG-lane group has its own copy of the sums, so the
 // lanes of a step mostly meet different words.
 // ---------------------------------------------------------------------------
+constexpr int LIMB_ADDITIONS = 64;
+constexpr long long LIMB_MAX = (1LL << 49) - 1;
+static_assert(LIMB_ADDITIONS * 0xffffffLL <= 0xffffffffLL, "low limb");
+static_assert(
+    LIMB_ADDITIONS * (LIMB_MAX >> 24) <= 0x7fffffffLL && LIMB_ADDITIONS * (-LIMB_MAX >> 24) >= -0x80000000LL, "high limb");
+
 template <typename Real> struct alignas(2 * sizeof(Real)) Vec2 {
     Real a, b;
 };
@@ -1289,8 +1295,8 @@ template <typename Real> struct alignas(2 * sizeof(Real)) Vec2 {
 // The rows of one work item, one instance per warp.
 template <typename Real, bool DX, bool DP, bool INTERP, int RG> struct alignas(16) WalkRows {
     static constexpr int FIELDS = (DX ? 3 : 0) + (DP ? 3 : 0);
-    // tiles between two flushes of the row sums: at most 64 additions to a word
-    static constexpr int FLUSH_TILES = 64 / RG;
+    // tiles between two flushes of the row sums: at most LIMB_ADDITIONS to a word
+    static constexpr int FLUSH_TILES = LIMB_ADDITIONS / RG;
     // coordinates row by row for the distance pass, and as pairs for the walk
     Real x[RG], y[RG], z[RG];
     Vec2<Real> xy[RG], zq[RG], se[RG], wd[RG]; // (x, y), (z, q), (sig, eps), (w, dw/dlambda)
@@ -1326,8 +1332,9 @@ template <typename Real> __device__ __forceinline__ WalkBox<Real> walk_box(const
     return b;
 }
 
-// A fixed-point value that the limbs hold.
-template <typename Real> __device__ __forceinline__ bool fits_limbs(Real y) { return fabs(y) < static_cast<Real>(0x1p49); }
+// A value that the limbs hold once it is rounded: |y| < LIMB_MAX rounds to at most
+// LIMB_MAX in FP64; in FP32, where LIMB_MAX is 2^49, the next smaller y is an integer.
+template <typename Real> __device__ __forceinline__ bool fits_limbs(Real y) { return fabs(y) < static_cast<Real>(LIMB_MAX); }
 
 __device__ __forceinline__ void limbs_add(unsigned (*acc)[TILE], int field, int word, unsigned long long v) {
     atomicAdd(&acc[2 * field][word], static_cast<unsigned>(v) & 0xffffffu);

@@ -193,3 +193,24 @@ def test_an_atom_without_a_position_pairs_with_none(n, value):
                 _assert_same((dx[rest], dp.reshape(N, 3)[rest].reshape(-1), dl, u), want)
             else:
                 np.testing.assert_allclose(fixed_to_float(u), fixed_to_float(want[3]), rtol=1e-5)
+
+
+@pytest.mark.parametrize("interpolated", [False, True])
+def test_pair_list_outputs_do_not_carry_over(interpolated):
+    """A pair list clears the accumulators of the outputs it was asked for; calls
+    with other outputs and windows in between find all of them at zero."""
+    x, p, box, plane, offset = _case(300, 1, 0)
+    if interpolated:
+        p = np.concatenate([p, f32_round(1.2 * p)])
+    rng = np.random.default_rng(3)
+    pairs = np.array([c for c in rng.integers(0, 300, size=(900, 2)) if c[0] != c[1]], dtype=np.int32)
+    cls = P.NonbondedPairListInterpolated if interpolated else P.NonbondedPairList
+    make = lambda: cls(pairs, np.ones((len(pairs), 2)), plane, offset, 2.0, 1.2).unbound_impl(np.float32)
+    want = _fixed(make(), x, p, box, 0.3)
+    impl = make()
+    flags = [f for f in P.all_flag_combinations() if any(f)]
+    for k in rng.permutation(np.repeat(np.arange(len(flags)), 3)):
+        _assert_same(_fixed(impl, x, p, box, 0.3, flags[k]), [w if f else None for w, f in zip(want, flags[k])])
+        if k % 4 == 0:
+            multi = impl.execute_windows_fixed(x, p, box, np.array([0.3, 0.9]))
+            _assert_same([multi[j][0] if j < 2 else multi[j][0].sum(dtype=np.uint64) for j in range(4)], want)

@@ -448,6 +448,22 @@ class NonbondedPotential : public PotentialBase {
     // Elements of one accumulator block (8 or 11 arrays of S slots).
     size_t acc_block_elems() const { return (size_t)S_ * (split_pair_dp_ ? 11 : 8); }
 
+    // The accumulators that a call with these outputs adds into (first element,
+    // number): one window's are x y z, q sig eps, u, dl, then the scaled pairs' q sig
+    // eps. A pair list clears them after the call; clearing all of them costs forces
+    // of 1,000,000 atoms 77.1 us instead of 70.0.
+    std::pair<size_t, size_t> acc_used(int K, int kidx) const {
+        if (K > 1) {
+            return {0, acc_block_elems() * (1 + K)};
+        }
+        const size_t S = S_;
+        const size_t first = (kidx & 4) ? 0 : (kidx & 1) ? 3 * S : (kidx & 8) ? 6 * S : 7 * S;
+        const size_t last = (kidx & 1) && split_pair_dp_
+                                ? 11 * S
+                                : (kidx & 2) ? 8 * S : (kidx & 8) ? 7 * S : (kidx & 1) ? 6 * S : 3 * S;
+        return {first, last - first};
+    }
+
     // Staging and accumulator capacity for K windows: K staged copies of the
     // slots and, for K > 1, the shared block plus one block per window.
     void ensure_windows(int K) {
@@ -659,8 +675,8 @@ class NonbondedPotential : public PotentialBase {
             launch_dependent(k_finalize, dim3(fgrid), dim3(tpb), 0, stream, fa);
             CK(cudaPeekAtLastError());
             if (!has_nblist_) { // else k_build_tiles clears them before the pair kernel
-                CK(cudaMemsetAsync(
-                    acc_.p, 0, acc_block_elems() * (K > 1 ? 1 + K : 1) * sizeof(unsigned long long), stream));
+                const auto used = acc_used(K, kidx);
+                CK(cudaMemsetAsync(acc_.p + used.first, 0, used.second * sizeof(unsigned long long), stream));
             }
             stage_end(TMNB_STAGE_FINALIZE, stream);
         }
@@ -767,22 +783,15 @@ class NonbondedPotential : public PotentialBase {
             launch_dependent(
                 k_stage_blocks, dim3((RB_ + 3) / 4), dim3(128), 0, stream, sa, pa, to, cst);
         }
-        // the accumulators this call adds into: the arrays of its outputs (one
-        // window: x y z, q sig eps, u, dl, then the scaled pairs' q sig eps)
-        size_t first = 0, last = acc_block_elems() * (K > 1 ? 1 + K : 1);
-        if (K == 1) {
-            const size_t S = S_;
-            first = (kidx & 4) ? 0 : (kidx & 1) ? 3 * S : (kidx & 8) ? 6 * S : 7 * S;
-            last = (kidx & 1) && split_pair_dp_ ? 11 * S
-                                                : (kidx & 2) ? 8 * S : (kidx & 8) ? 7 * S : (kidx & 1) ? 6 * S : 3 * S;
-        }
-        const size_t n_clear = kidx == 0 ? 0 : last - first;
+        const auto used = acc_used(K, kidx);
+        const size_t n_clear = kidx == 0 ? 0 : used.second;
         // one CTA per row group; more where few row groups (an interaction
         // group's) would clear for long
         const size_t ctas = std::max<size_t>(
             n_row_blocks_, std::min<size_t>(num_sms(), (n_clear + TB_WARPS * 32 - 1) / (TB_WARPS * 32)));
         launch_dependent(
-            k_build_tiles, dim3((unsigned)ctas), dim3(TB_WARPS * 32), 0, stream, ta, acc_.p + first, n_clear, state_.p);
+            k_build_tiles, dim3((unsigned)ctas), dim3(TB_WARPS * 32), 0, stream, ta, acc_.p + used.first, n_clear,
+            state_.p);
         CK(cudaPeekAtLastError());
     }
 

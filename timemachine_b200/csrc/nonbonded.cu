@@ -430,13 +430,16 @@ class NonbondedPotential : public PotentialBase {
     // Tiles per work item of a list built by a K-window call: few enough that
     // every resident warp has work and the last items end together, as many as
     // that allows (each item loads and flushes its rows once). Measured on B200,
-    // us per call, 1 / 2 / 4 tiles (forces) and 2 / 4 / 8 (12 windows):
-    // 2,500 atoms 26.1 / 30.8 / 40.2 and 53.0 / 64.2 / 86.5; 10,000: 46.5 / 48.7 /
-    // 55.0 and 83.3 / 87.0 / 101; 22,840: 81.2 / 79.6 / 84.8 and 136.1 / 137.2 /
-    // 147; 98,000: 273 / 252 / 249 and 455 / 436 / 441.
+    // us per call at 1 / 2 / 4 tiles, forces and 12 windows: 2,500 atoms 23.9 / 28.2 /
+    // 37.6 and 37.9 / 41.7 / 52.2; 5,000: 29.7 / 33.0 / 40.0 and 47.0 / 46.8 / 58.9;
+    // 16,000: 55.9 / 56.0 / 62.7 and 90.1 / 86.3 / 92.7; 22,840: 73.4 / 71.0 / 74.2 and
+    // 120.5 / 112.9 / 117.5; 40,000: 117.7 / 111.1 / 112.7 and 192.9 / 178.5 / 180.2;
+    // 98,000: 259.6 / 238.3 / 234.2 and 440 / 403 / 393. Interaction groups, by their
+    // rows, forces and 8 windows: 400 rows 19.2 / 24.4 / 33.8 and 39.9 / 41.6 / 52.2;
+    // 2,000: 20.5 / 24.2 / 31.0 and 39.8 / 43.2 / 52.3; 6,000: 26.1 / 27.1 / 33.2 and
+    // 44.1 / 46.3 / 53.5; 30,000: 50.0 / 49.4 / 53.1 and 111.6 / 111.7 / 116.6.
     int list_chunk(int K) const {
-        // a group's rows reach about twice the columns of as many all-pairs rows
-        const long long n = kind_ == Kind::Group ? 2LL * NR_ : S_;
+        const int n = row_end();
         if (K > 1) {
             return n < 4000 ? 1 : (n < 40000 ? 2 : 4);
         }
@@ -1051,7 +1054,9 @@ namespace tmb {
 // copy together with the error word; larger ones go straight to the caller's
 // arrays. Measured on B200 against four clears, five copies back and the
 // decoding in numpy: 900 atoms, all outputs 157 -> 84 us per call; 4 frames x 6
-// windows of 5,000 atoms 2,720 -> 1,054.
+// windows of 5,000 atoms 2,720 -> 1,054. The line, all outputs of one window, copies
+// of their own / one staged copy: 120 KB 114 / 106 us, 240 KB 142 / 143, 384 KB 168 /
+// 188, 1.1 MB 311 / 390.
 constexpr size_t HOST_STAGE = 256 * 1024;
 
 void PotentialBase::execute_decoded_host(

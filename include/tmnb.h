@@ -320,7 +320,9 @@ tmnb_status tmnb_potential_copy_nblist(
 
 /* Instrumentation (no reference counterpart): CUDA events around every
  * stage of a call on the launching stream, and the duration of the stage's
- * last launch (synchronises on its end event). Stages: */
+ * last launch (synchronises on its end event). While it is on, small calls (up
+ * to 8,192 atoms x windows), whose preparation, slot order and staging are
+ * otherwise one kernel, run them as the kernels of large calls. Stages: */
 #define TMNB_STAGE_PREPARE 0  /* rebuild check, box checks, staging (k_check_prepare) */
 #define TMNB_STAGE_REBUILD 1  /* neighbour-list rebuild chain (returns at once when none is due) */
 #define TMNB_STAGE_PAIR 2     /* pair kernel */

@@ -418,7 +418,7 @@ __device__ __forceinline__ PairArgs pair_args(const Rep &r) {
 // 395 -> 354. Without derivatives (forces, energy) two walks are no faster (64 of
 // 1,500: 192 / 190 and 139 / 141; 4 of 22,840: 249 / 254 and 167 / 181).
 template <bool U, bool DX, bool DL, bool DP, int RG>
-__global__ void __launch_bounds__(128, DP ? 5 : (pair_min_ctas<float, U, DX, DL, DP, false, RG>()))
+__global__ void __launch_bounds__(128, DP ? 5 : PAIR_MIN_CTAS<float>)
     k_b_pair(const Rep *__restrict__ reps, int R, const int *__restrict__ prefix, int *counter) {
     __shared__ WalkRows<float, DX, DP, false, RG> rows[4];
     WalkRows<float, DX, DP, false, RG> &sm = rows[threadIdx.x >> 5];

@@ -35,18 +35,6 @@ namespace tmb {
 constexpr unsigned FULL_MASK = 0xffffffffu;
 constexpr int TILE = 32;
 
-// CTAs per SM that the pair kernel's registers must fit: force / energy
-// outputs, with parameter derivatives, FP64.
-#ifndef TMNB_WALK_CTAS
-#define TMNB_WALK_CTAS 6
-#endif
-#ifndef TMNB_WALK_CTAS_ALL
-#define TMNB_WALK_CTAS_ALL 6
-#endif
-#ifndef TMNB_WALK_CTAS_F64
-#define TMNB_WALK_CTAS_F64 5
-#endif
-
 // Sticky device-side state of one potential instance.
 struct DevState {
     int rebuild;          // 1: the neighbour list must be rebuilt in this evaluation
@@ -874,7 +862,8 @@ __device__ __forceinline__ int tb_emit(TileBuildSmem &sm, const TileArgs &a, int
 // Up to 32 column atoms (one per lane, `active`; slot in q.w) against the row
 // atoms: those within the list radius of one are collected with their key.
 __device__ __forceinline__ void tb_test_columns(
-    TileBuildSmem &sm, const TileArgs &a, const float4 q, const bool active, const bool shifted, const float r2, const float Lx, const float Ly, const float Lz, const float iLx, const float iLy, const float iLz) {
+    TileBuildSmem &sm, const TileArgs &a, const float4 q, const bool active, const bool shifted, const float r2,
+    const float Lx, const float Ly, const float Lz, const float iLx, const float iLy, const float iLz) {
     const int lane = threadIdx.x & 31;
     const float rc2 = a.cutoff * a.cutoff;
     float d2_min = 3.0e38f;
@@ -1169,9 +1158,6 @@ static __global__ void __launch_bounds__(TB_WARPS * 32, TMNB_TB_CTAS) k_build_ti
     build_tiles_cta(a, blockIdx.x, state);
 }
 
-// Clears the rebuild flag when no neighbour list exists (pair lists only).
-static __global__ void k_clear_rebuild(DevState *state) { state->rebuild = 0; }
-
 // ---------------------------------------------------------------------------
 // Pair kernel.
 // ---------------------------------------------------------------------------
@@ -1255,14 +1241,14 @@ template <> struct Staged<double> {
 // Tile walk: the pairs of a tile (RG rows x 32 columns) that lie within the
 // cutoff, and only those.
 //
-// What bounds it: instruction issue and the shared-memory pipe (ncu, forces at
-// 22,840 atoms: 64 % of issue slots, 28.6 of 32 lanes per instruction, 65 % of
-// the L1 / shared wavefronts; DRAM idle). The sweep of every row x column that
-// this replaced issued 69.8 M warp instructions there, the walk 43.4 M. Kernel
+// What bounds it (ncu, forces at 22,840 atoms): no pipe by itself. 64 % of the issue
+// slots are taken, 28.6 of 32 lanes per instruction, 65 % of the L1 / shared
+// wavefronts, DRAM idle; 34 % of the warps are active and wait longest for loaded
+// columns (long_scoreboard, 2.2 cycles per issue). The sweep of every row x column
+// that this replaced issued 69.8 M warp instructions there, the walk 43.4 M. Kernel
 // times on B200 under ncu, before -> after, bit-identical: forces 92.3 -> 69.2 us,
-// all outputs of 12 windows 154 -> 104 (FP64 410 -> 209), batch of 64 replicas
-// 3.04 -> 2.56 ms. 7 or 8 CTAs/SM instead of 6 change nothing; loading the next
-// tile's columns ahead costs 2 to 6 %.
+// all outputs of 12 windows 154 -> 104 (FP64 410 -> 209). CTAs per SM: PAIR_MIN_CTAS;
+// loading the next tile's columns ahead costs 2 to 6 %.
 //
 // Lane l owns column l of the tile: its atom and its sums stay in registers.
 // The tile's rows are staged in shared memory once per work item. A tile takes
@@ -2024,18 +2010,11 @@ __device__ __forceinline__ int next_unit(int *counter, int n_first, int lane) {
     return n_first + __shfl_sync(FULL_MASK, v, 0);
 }
 
-// CTAs per SM the compiler must fit for each pair-kernel variant (its
-// register budget).
-template <typename Real, bool U, bool DX, bool DL, bool DP, bool INTERP, int RG>
-constexpr int pair_min_ctas() {
-    if (sizeof(Real) != 4) {
-        return TMNB_WALK_CTAS_F64;
-    }
-    if (DP) {
-        return TMNB_WALK_CTAS_ALL;
-    }
-    return TMNB_WALK_CTAS;
-}
+// CTAs per SM the compiler must fit the pair kernel to (its register budget). FP32 on
+// B200, us per call at 5 / 6 / 7 / 8, 22,840 and 98,000 atoms: forces 75.1 / 71.2 / 69.7 /
+// 68.8 and 256 / 239 / 231 / 225, all outputs 96.7 / 93.1 / 96.2 / 103.7 and 331 / 314 /
+// 322 / 347, 12 windows 117 / 112 / 117 / 126 and 416 / 392 / 407 / 437.
+template <typename Real> constexpr int PAIR_MIN_CTAS = sizeof(Real) == 4 ? 6 : 5;
 
 // Persistent pair kernel over dynamically scheduled work units:
 //   [0, n_items)                 tile work items (row group, first tile, count);
@@ -2045,7 +2024,7 @@ constexpr int pair_min_ctas() {
 // into the shared accumulator block; each (tile, window) unit adds into the
 // window's block; a lambda-dependent scaled pair is evaluated for every window.
 template <typename Real, bool U, bool DX, bool DL, bool DP, bool INTERP, bool MULTI, int RG = TILE>
-__global__ void __launch_bounds__(128, (pair_min_ctas<Real, U, DX, DL, DP, INTERP, RG>())) k_pair(PairArgs a) {
+__global__ void __launch_bounds__(128, PAIR_MIN_CTAS<Real>) k_pair(PairArgs a) {
     __shared__ WalkRows<Real, DX, DP, INTERP, RG> rows[4];
     grid_dependency_wait();
     if (a.state->error) {

@@ -176,9 +176,6 @@ template <typename Real> __device__ __forceinline__ Real sum_of_products_rn(Real
     return fadd(fmul(a, b), fmul(c, d));
 }
 
-// acc + a*b with the reference's fused rounding
-template <typename Real> __device__ __forceinline__ Real mul_add(Real a, Real b, Real acc) { return ffma(a, b, acc); }
-
 __device__ __forceinline__ float inv_sqrt(float x) { return rsqrtf(x); }
 __device__ __forceinline__ double inv_sqrt(double x) { return rsqrt(x); }
 

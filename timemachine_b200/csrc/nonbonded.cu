@@ -234,7 +234,9 @@ class NonbondedPotential : public PotentialBase {
     // CUDA events around every stage of a call (on the launching stream):
     // TMNB_STAGE_PREPARE (k_check_prepare), _REBUILD (the rebuild-chain
     // kernels, which return at once when no rebuild is due, and the clearing of
-    // the accumulators), _PAIR (k_pair), _FINALIZE (k_finalize).
+    // the accumulators), _PAIR (k_pair), _FINALIZE (k_finalize). Calls of up to
+    // CLUSTER_PREPARE_MAX staged slots, whose front is one kernel, run it as
+    // k_check_prepare, k_order_slots and k_stage_blocks while timing is on.
     void enable_timing(bool on) {
         if (on && !timing_) {
             for (auto &e : ev_) {
@@ -645,7 +647,7 @@ class NonbondedPotential : public PotentialBase {
             CK(cudaPeekAtLastError());
             stage_end(TMNB_STAGE_PAIR, stream);
             if (fuse_ & FUSE_KEEP_FORCES) {
-                return; // the integrator kernel reads and clears the accumulators
+                return; // the integrator kernel reads the accumulators, the next tile build clears them
             }
 
             FinalizeArgs fa;

@@ -192,3 +192,26 @@ def test_all_outputs_of_small_replicas_cost_little_more_than_forces():
     forces, everything = ms(du_dp=False, du_dl=False, u=False), ms()
     print(f"forces {forces:.4f} ms, all outputs {everything:.4f} ms, ratio {everything / forces:.2f}")
     assert everything < 1.7 * forces
+
+
+@pytest.mark.parametrize("rows", [8, 16, 32])
+def test_long_items_equal_single_system_evaluation(rows):
+    """64 tiles per work item: the row sums are flushed in the middle of items, and
+    would not fit their limbs otherwise (equal charges and a slowly decaying
+    interaction: most of a row's charge derivatives lie between 2^47 and 2^49)."""
+    s, lam = testsystems.system_of_size(5200, seed=103), 0.4
+    s.beta = 0.5
+    s.params[:, 0] = 7400.0
+    b = ReplicaBatch()
+    b.set_tuning(chunk=64, rows=rows)
+    rid = b.add(s, lam)
+    b.evaluate()
+    tiles, items, _ = b.stats(rid)
+    assert tiles > 16 * items
+    got, want = b.result_fixed(rid), _single_fixed(s, lam)
+    np.testing.assert_array_equal(got[0], want[0])
+    np.testing.assert_array_equal(got[1], want[1].reshape(-1, 3))
+    assert got[2].sum(dtype=np.uint64) == want[2].sum(dtype=np.uint64)
+    assert got[3].sum(dtype=np.uint64) == want[3].sum(dtype=np.uint64)
+    # the high limbs of a row (one for each of the 32 / rows copies) hold 2^31 << 24
+    assert got[1][:, 0].view(np.int64).max() > (32 // rows) * 2.0**55

@@ -94,9 +94,10 @@ def test_dense_group_fills_the_column_buffer(interpolated):
     assert all(len(np.unique(t)) == len(t) for t in got)
 
 
-@pytest.mark.parametrize("n", [255, 8192, 8193, 32768, 32769])
+@pytest.mark.parametrize("n", [255, 8192, 8193, 32768, 32769, 131105])
 def test_rebuild_paths(n):
-    """Sizes at the edges of the three ways a call prepares and sorts: the list
+    """Sizes at the edges of the three ways a call prepares and sorts, and one whose
+    column blocks the tile build goes through in two passes (4,096 each): the list
     that each leaves gives the pair list's sums, with and without the Hilbert
     order, after the atoms have moved and with other windows per call."""
     rng = np.random.default_rng(n)
@@ -214,3 +215,23 @@ def test_pair_list_outputs_do_not_carry_over(interpolated):
         if k % 4 == 0:
             multi = impl.execute_windows_fixed(x, p, box, np.array([0.3, 0.9]))
             _assert_same([multi[j][0] if j < 2 else multi[j][0].sum(dtype=np.uint64) for j in range(4)], want)
+
+
+def test_long_items_flush_between_tiles_left_out():
+    """32 rows and four tiles per item (several windows, from 40,000 atoms on): the row
+    sums are flushed in the middle of an item, whose lambda-dependent tiles are left
+    out and evaluated per window. Equal to 16 rows, one window at a time."""
+    s = testsystems.system_of_size(40500, seed=11, n_ligand=40)
+    x, p = f32_round(s.x), f32_round(s.params)
+    offset = s.lambda_offset_idxs.copy()
+    offset[np.random.default_rng(4).choice(s.N, 30, replace=False)] = 1  # lambda-dependent tiles in many items
+    lams = np.array([0.2, 0.7])
+    impl = P.NonbondedAllPairs(s.lambda_plane_idxs, offset, s.beta, s.cutoff).unbound_impl(np.float32)
+    one = P.NonbondedAllPairs(s.lambda_plane_idxs, offset, s.beta, s.cutoff).unbound_impl(np.float32)
+    impl.set_tile_rows(32)
+    got = impl.execute_windows_fixed(x, p, s.box, lams)
+    tiles, items, _ = impl.nblist_stats()
+    assert tiles > 3 * items  # most items hold four
+    for k, lam in enumerate(lams):
+        want = _fixed(one, x, p, s.box, lam)
+        _assert_same([got[j][k] if j < 2 else got[j][k].sum(dtype=np.uint64) for j in range(4)], want)

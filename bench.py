@@ -99,8 +99,8 @@ FLOPS_PER_PAIR = _table_sum("distance", "electrostatics", "forces", "charge deri
 FLOPS_PER_LJ_PAIR = _table_sum("lennard_jones (both atoms carry epsilon)")
 FLOPS_PER_ALCH_PAIR = _table_sum("lambda-dependent pair (an atom with a nonzero lambda offset)")
 # DRAM bytes (read + write) of one 12-window pair-kernel launch on this
-# workload, from an ncu capture of the same command (13.4 MB read, 0 written)
-PAIR_LAUNCH_DRAM_BYTES = 13.4e6
+# workload, from an ncu capture of the same command (13.2 MB read, 0 written)
+PAIR_LAUNCH_DRAM_BYTES = 13.2e6
 # stages of a call timed by tmnb_potential_last_stage_ms
 STAGE_PREPARE, STAGE_REBUILD, STAGE_PAIR, STAGE_FINALIZE = 0, 1, 2, 3
 
@@ -567,22 +567,20 @@ def run_tmnb(args, world, rank, local):
     if rank == 0:
         errors = output_errors(s, x, p, float(lambdas[6]), {"f32": f32_fixed, "f64": f64_fixed})
 
-    # end to end through the C-ABI host entry (pinned host buffers, copies inside)
+    # end to end through the host entry that Potential.execute_windows calls (pinned
+    # host buffers, copies and decoding inside)
     hx = torch.as_tensor(x).pin_memory().numpy()
     hp = torch.as_tensor(p).pin_memory().numpy()
     hb = torch.as_tensor(s.box).pin_memory().numpy()
     hl = torch.as_tensor(lambdas).pin_memory().numpy()
     outs = [
-        torch.zeros(sh, dtype=torch.int64).pin_memory().numpy().view(np.uint64)
-        for sh in [(K, N, 3), (K, p.size), (K, N), (K, N)]
+        torch.zeros(sh, dtype=torch.float64).pin_memory().numpy() for sh in [(K, N, 3), (K, p.size), (K,), (K,)]
     ]
 
     def host_step():
         _lib.check(
-            lib.tmnb_potential_execute_windows_host(
-                impl.handle, N, p.size, hx.ctypes.data_as(ctypes.c_void_p), hp.ctypes.data_as(ctypes.c_void_p),
-                hb.ctypes.data_as(ctypes.c_void_p), K, hl.ctypes.data_as(ctypes.c_void_p),
-                *[o.ctypes.data_as(ctypes.c_void_p) for o in outs],
+            lib.tmnb_potential_execute_decoded_host(
+                impl.handle, 1, N, 1, p.size, K, *[a.ctypes.data_as(ctypes.c_void_p) for a in (hx, hp, hb, hl, *outs)]
             )
         )
 
@@ -600,8 +598,9 @@ def run_tmnb(args, world, rank, local):
     h2d = hx.nbytes + hp.nbytes + hb.nbytes + hl.nbytes
     d2h = sum(o.nbytes for o in outs)
 
-    # check/prepare, 5 rebuild-chain kernels (returning at once unless rebuilding), dep tiles, pair, finalize
-    launches_per_step = 9
+    # check/prepare, 3 rebuild-chain kernels (the order and staging return at once unless
+    # rebuilding, the tile build clears the accumulators), dep tiles, pair, finalize
+    launches_per_step = 7
     result = {
         "metric": "nonbonded evals/s at 22,840 atoms (u, du_dx, du_dp, du_dl; 12 lambda windows per step)",
         "value": value,
@@ -636,7 +635,7 @@ def run_tmnb(args, world, rank, local):
             "unit": "TFLOP/s",
             "frac": achieved / peak.value,
             # dram__bytes_read.sum + dram__bytes_write.sum of one launch of this kernel on
-            # this workload (ncu capture, k_pair_12windows_water_ligand_22840.md under
+            # this workload (ncu capture, k_pair_walk_22840.md under
             # profiles/): the working set stays in L2, DRAM is not the bound
             "traffic": PAIR_LAUNCH_DRAM_BYTES,
             "traffic_unit": "bytes per launch",

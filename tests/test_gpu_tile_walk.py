@@ -8,8 +8,10 @@ column buffer."""
 
 import numpy as np
 import pytest
+import torch
 from scipy.spatial import cKDTree
 
+from tests.gpu_helpers import to_dev
 from tests.helpers import f32_round, random_params
 from timemachine_b200 import potentials as P
 from timemachine_b200 import testsystems
@@ -235,3 +237,25 @@ def test_long_items_flush_between_tiles_left_out():
     for k, lam in enumerate(lams):
         want = _fixed(one, x, p, s.box, lam)
         _assert_same([got[j][k] if j < 2 else got[j][k].sum(dtype=np.uint64) for j in range(4)], want)
+
+
+def test_the_first_slots_are_tried_again():
+    """After a wide row group 1,000 rebuilds keep the plain order, then the atoms take
+    the first slots once more."""
+    s = testsystems.system_of_size(3000, seed=2, n_ligand=20)
+    offset = np.zeros(s.N, np.int32)
+    offset[np.random.default_rng(1).choice(s.N, 64, replace=False)] = 1
+    impl = P.NonbondedAllPairs(np.zeros(s.N, np.int32), offset, s.beta, s.cutoff).unbound_impl(np.float32)
+    frames = [to_dev(s.x), to_dev(s.x + 0.3)]
+    p, box = to_dev(s.params).reshape(-1), to_dev(s.box)
+    out = torch.zeros((s.N, 3), dtype=torch.int64, device="cuda")
+    first = []
+    for k in range(1004):
+        impl.execute_device(frames[k % 2], p, box, 0.3, out)
+        if k in (0, 1, 2, 500, 999, 1000, 1001, 1002, 1003):
+            torch.cuda.synchronize()
+            perm, _, _ = impl.get_nblist()
+            if set(perm[:64]) == set(np.flatnonzero(offset)):
+                first.append(k)
+    assert impl.nblist_stats()[2] == 1004  # every call rebuilt
+    assert first == [0, 1001]

@@ -69,7 +69,7 @@ def test_all_pairs_equals_pair_list(n, rows, precision, images):
 @pytest.mark.parametrize("interpolated", [False, True])
 def test_dense_group_fills_the_column_buffer(interpolated):
     """16 + 3 row atoms with about 6,000 column atoms in reach: more than the
-    list builder sorts at once."""
+    list builder sorts; the others follow unsorted."""
     n, nr = 6019, 19
     rng = np.random.default_rng(5)
     edge = 3.0
@@ -259,3 +259,37 @@ def test_the_first_slots_are_tried_again():
                 first.append(k)
     assert impl.nblist_stats()[2] == 1004  # every call rebuilt
     assert first == [0, 1001]
+
+
+def test_rebuild_of_wide_lists_costs_one_pass():
+    """At 1.6 nm many row groups list more columns than the builder sorts. A
+    rebuilding energy call of 5,000 atoms took twice one that keeps its list before
+    the columns were sorted, 2.9 times when such a group was done again in rounds, and
+    takes 2.2 times now."""
+    n, edge, cutoff = 5000, 50.0 ** (1.0 / 3.0), 1.6
+    rng = np.random.default_rng(0)
+    g = (np.arange(18) + 0.5) * edge / 18
+    x = np.stack(np.meshgrid(g, g, g, indexing="ij"), axis=-1).reshape(-1, 3)
+    x = x[rng.choice(len(x), n, replace=False)] + rng.normal(scale=0.02, size=(n, 3))
+    p = np.stack([rng.normal(size=n), np.full(n, 0.15), np.where(np.arange(n) % 3 == 0, 0.8, 0.0)], axis=1)
+    zero = np.zeros(n, np.int32)
+    impl = P.NonbondedAllPairs(zero, zero, 2.0, cutoff).unbound_impl(np.float32)
+    frames = [to_dev(x), to_dev(x + 0.3)]
+    dp, box, u = to_dev(p).reshape(-1), to_dev(np.eye(3) * edge), torch.zeros(n, dtype=torch.int64, device="cuda")
+
+    def us(moving):
+        best = np.inf
+        for _ in range(6):
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            start.record()
+            for k in range(20):
+                impl.execute_device(frames[k % 2 if moving else 0], dp, box, 0.3, None, None, None, u)
+            end.record()
+            end.synchronize()
+            best = min(best, start.elapsed_time(end) / 20 * 1e3)
+        return best
+
+    kept, rebuilt = us(False), us(True)
+    assert max(len(t) for t in impl.get_nblist()[1]) > 3072
+    print(f"list kept {kept:.1f} us, rebuilt {rebuilt:.1f} us")
+    assert rebuilt < 2.7 * kept

@@ -308,15 +308,15 @@ __device__ __forceinline__ unsigned hilbert_index_3d(unsigned x, unsigned y, uns
 
 // Atoms with a lambda offset take the first slots, in the order of their indices
 // (a ligand's follow its bonds), as long as their row groups stay compact. A group
-// with atoms of two places lists the columns around both, and the rebuild waits
-// for its one CTA. The tile build measures the groups: when the half diagonal of
-// one's box exceeds SITE_EXTENT cutoffs, or its columns do not fit the buffer, the
-// next SITE_RETRY rebuilds keep the plain order, and then the rule is tried again.
-// Measured on B200 at 22,840 atoms, us per call with a rebuild, those atoms first
-// wherever they are / plain order / this rule: forces, one ligand 130 / 128 / 129,
-// with a distant ion 184 / 129 / 127, two ligands 240 / 129 / 128, 1 % of the atoms
-// anywhere 287 / 133 / 132; 12 windows 189 / 198 / 190, 243 / 202 / 203, 304 / 214 /
-// 214, 390 / 391 / 392. Two places 1.5 nm apart (10,000 atoms) 85 / 76 / 78.
+// with atoms of two places goes through the columns around both, and the rebuild
+// waits for its one CTA. The tile build measures the groups: when the half diagonal
+// of one's box exceeds SITE_EXTENT cutoffs, the next SITE_RETRY rebuilds keep the
+// plain order, and then the rule is tried again. Measured on B200 at 22,840 atoms,
+// us per call with a rebuild, those atoms first wherever they are / plain order / this
+// rule: forces, one ligand 130 / 128 / 130, with a distant ion 167 / 129 / 128, two
+// ligands 162 / 129 / 129, 1 % of the atoms anywhere 163 / 133 / 132; 12 windows (more
+// than one such atom in 128: first wherever they are) 189 / 198 / 189, 227 / 202 / 203,
+// 226 / 214 / 214, 274 / 391 / 274.
 constexpr unsigned SITE_KEY = 0xffffffffu; // instead of a cell's
 constexpr float SITE_EXTENT = 1.0f;
 constexpr int SITE_RETRY = 1000;
@@ -761,12 +761,12 @@ __host__ __device__ __forceinline__ long long tile_base(const TileArgs &a, int g
 }
 
 constexpr int TB_WARPS = 8;
-// Column atoms the CTA holds before it sorts them into tiles. Groups of 16
-// rows list about 900 atoms at 100 atoms per nm^3; a group that lists more
-// than fit is done again in rounds of TB_ROUND blocks, each followed by a
-// check, and a nearly full buffer is sorted and its whole tiles are written.
+// Column atoms of a group that the CTA sorts into its tiles; the ones found after
+// them follow in the order they were found. Groups of 16 rows list up to 2,000 at 100
+// atoms per nm^3 and 1.2 nm, up to 3,500 at 1.6 nm. Measured on B200, us of an energy
+// call with a rebuild, 5,000 atoms at 1.6 nm: 78 (doing such a group again, in rounds
+// of 32 column blocks, 106; room for 4,608 columns 80); 20,000 atoms 150 (195; 151).
 constexpr int TB_COLS = 3072;
-constexpr int TB_ROUND = 32;
 constexpr int TB_WINDOWS = 16; // box tests per thread before the atoms are gone through
 // sort keys: lambda dependence x Lennard-Jones x 33 row counts
 constexpr int TB_KEYS = 2 * 2 * 33;
@@ -789,19 +789,17 @@ struct TileBuildSmem {
     float4 row_box[2]; // the row group's box: centre, half-extent
     unsigned cols[TB_COLS];
     unsigned char keys[TB_COLS];
-    unsigned rem_cols[TILE];
-    unsigned char rem_keys[TILE];
     int bins[TB_KEYS]; // columns of each key, then the next position of each key
-    int n_cols;
+    int n_cols; // all of the group's
     float4 queue[TB_WARPS][2 * TILE]; // column atoms in reach of the group's box: position, slot
     unsigned passing[TB_WINDOWS * TB_WARPS]; // column blocks that pass the box test, one bit each
     int is_last;
 };
 
-// Sorts the CTA's n collected columns by key and writes them as tiles from
-// first_tile on: all of them (the last tile padded with S) when `last`,
-// else the whole tiles, keeping the rest collected. Returns the tiles written.
-__device__ __forceinline__ int tb_emit(TileBuildSmem &sm, const TileArgs &a, int n, long long first_tile, bool last) {
+// Writes the group's n columns as tiles from dst on: the collected ones sorted by
+// key; those after them are there already. The last tile is padded with S.
+// Returns the tiles.
+__device__ __forceinline__ int tb_emit(TileBuildSmem &sm, const TileArgs &a, const int n, unsigned *dst) {
     const int lane = threadIdx.x & 31;
     if (threadIdx.x < TILE) {
         constexpr int PER = (TB_KEYS + TILE - 1) / TILE;
@@ -826,44 +824,24 @@ __device__ __forceinline__ int tb_emit(TileBuildSmem &sm, const TileArgs &a, int
         }
     }
     __syncthreads();
-    const int n_out = last ? (n + TILE - 1) / TILE * TILE : n / TILE * TILE;
-    unsigned *dst = a.tile_cols + first_tile * TILE;
-    for (int k = threadIdx.x; k < n; k += TB_WARPS * 32) {
-        const int pos = atomicAdd(&sm.bins[sm.keys[k]], 1);
-        if (pos < n_out) {
-            dst[pos] = sm.cols[k];
-        } else {
-            sm.rem_cols[pos - n_out] = sm.cols[k];
-            sm.rem_keys[pos - n_out] = sm.keys[k];
-        }
+    for (int k = threadIdx.x; k < min(n, TB_COLS); k += TB_WARPS * 32) {
+        dst[atomicAdd(&sm.bins[sm.keys[k]], 1)] = sm.cols[k];
     }
+    const int n_out = (n + TILE - 1) / TILE * TILE;
     if (n + (int)threadIdx.x < n_out) {
         dst[n + threadIdx.x] = (unsigned)a.S;
     }
     __syncthreads();
-    if (!last) {
-        for (int k = threadIdx.x; k < TB_KEYS; k += TB_WARPS * 32) {
-            sm.bins[k] = 0;
-        }
-        __syncthreads();
-        if ((int)threadIdx.x < n - n_out) {
-            sm.cols[threadIdx.x] = sm.rem_cols[threadIdx.x];
-            sm.keys[threadIdx.x] = sm.rem_keys[threadIdx.x];
-            atomicAdd(&sm.bins[sm.rem_keys[threadIdx.x]], 1);
-        }
-        if (threadIdx.x == 0) {
-            sm.n_cols = n - n_out;
-        }
-        __syncthreads();
-    }
     return n_out / TILE;
 }
 
 // Up to 32 column atoms (one per lane, `active`; slot in q.w) against the row
-// atoms: those within the list radius of one are collected with their key.
+// atoms: those within the list radius of one are collected with their key, or go
+// to their place among the group's columns (dst) where TB_COLS are collected.
 __device__ __forceinline__ void tb_test_columns(
     TileBuildSmem &sm, const TileArgs &a, const float4 q, const bool active, const bool shifted, const float r2,
-    const float Lx, const float Ly, const float Lz, const float iLx, const float iLy, const float iLz) {
+    const float Lx, const float Ly, const float Lz, const float iLx, const float iLy, const float iLz,
+    unsigned *dst) {
     const int lane = threadIdx.x & 31;
     const float rc2 = a.cutoff * a.cutoff;
     float d2_min = 3.0e38f;
@@ -903,19 +881,14 @@ __device__ __forceinline__ void tb_test_columns(
         at = atomicAdd(&sm.n_cols, __popc(hmask));
     }
     at = __shfl_sync(FULL_MASK, at, 0) + __popc(hmask & ((1u << lane) - 1));
-    if (hit && at < TB_COLS) {
-        const int s = __float_as_int(q.w);
+    const int s = __float_as_int(q.w);
+    if (hit && at >= TB_COLS) {
+        dst[at] = (unsigned)s;
+    } else if (hit) {
         const int key = (a.lamdep[s] ? 0 : 66) + (a.prm[s].z != 0.f ? 0 : 33) + 32 - near;
         sm.cols[at] = (unsigned)s;
         sm.keys[at] = (unsigned char)key;
         atomicAdd(&sm.bins[key], 1);
-    }
-}
-
-// Row group at row_first is wider than the rule for a site's atoms allows (one thread).
-__device__ __forceinline__ void site_too_wide(const TileArgs &a, const int row_first, DevState *state) {
-    if (row_first < a.n_site && *(volatile int *)&state->plain_order == 0) {
-        state->plain_order = SITE_RETRY + 1; // one of them is this rebuild, taken off at its end
     }
 }
 
@@ -959,8 +932,9 @@ __device__ __forceinline__ void build_tiles_cta(const TileArgs &a, const int rb,
                 0.5f * (mxz - mnz) * 1.000001f + 1e-6f, 0.f);
             const float ex = mxx - mnx, ey = mxy - mny, ez = mxz - mnz;
             const float widest = 2.0f * SITE_EXTENT * a.cutoff;
-            if (ex * ex + ey * ey + ez * ez > widest * widest) {
-                site_too_wide(a, row_first, state);
+            if (row_first < a.n_site && ex * ex + ey * ey + ez * ez > widest * widest &&
+                *(volatile int *)&state->plain_order == 0) {
+                state->plain_order = SITE_RETRY + 1; // one of them is this rebuild, taken off at its end
             }
         }
     }
@@ -1000,105 +974,79 @@ __device__ __forceinline__ void build_tiles_cta(const TileArgs &a, const int rb,
     // passing blocks cluster at nearby indices, so interleaving gives every warp
     // about as many, without ranking them.
     const int first_block = a.group ? a.cb_first : row_first / TILE;
-    int tiles = 0;  // tiles written so far (uniform over the CTA)
-    int n_have = 0; // columns collected (uniform over the CTA)
-    for (bool rounds = false;; rounds = true) {
-        const int round = rounds ? TB_ROUND : TB_WINDOWS * TB_WARPS * TILE;
-        for (int c0 = first_block; c0 < a.RB; c0 += round) {
-            const int c_end = min(a.RB, c0 + round);
-            const int windows = (c_end - c0 + TB_WARPS * TILE - 1) / (TB_WARPS * TILE);
-            for (int i = 0; i < windows; i++) {
-                const int cb = c0 + i * TB_WARPS * TILE + (int)threadIdx.x;
-                bool pass = false;
-                if (cb < c_end) {
-                    const float4 cc = a.bb_ctr[cb];
-                    const float4 ce = a.bb_ext[cb];
-                    const float dx = fmaxf(0.f, fabsf(wrap_delta(rc.x - cc.x, Lx, iLx)) - re.x - ce.x);
-                    const float dy = fmaxf(0.f, fabsf(wrap_delta(rc.y - cc.y, Ly, iLy)) - re.y - ce.y);
-                    const float dz = fmaxf(0.f, fabsf(wrap_delta(rc.z - cc.z, Lz, iLz)) - re.z - ce.z);
-                    pass = dx * dx + dy * dy + dz * dz < r2;
-                }
-                const unsigned m = __ballot_sync(FULL_MASK, pass);
-                if (lane == 0) {
-                    sm.passing[i * TB_WARPS + warp] = m;
-                }
+    unsigned *const dst = a.tile_cols + base_tile * TILE;
+    constexpr int PASS = TB_WINDOWS * TB_WARPS * TILE;
+    for (int c0 = first_block; c0 < a.RB; c0 += PASS) {
+        const int c_end = min(a.RB, c0 + PASS);
+        const int windows = (c_end - c0 + TB_WARPS * TILE - 1) / (TB_WARPS * TILE);
+        for (int i = 0; i < windows; i++) {
+            const int cb = c0 + i * TB_WARPS * TILE + (int)threadIdx.x;
+            bool pass = false;
+            if (cb < c_end) {
+                const float4 cc = a.bb_ctr[cb];
+                const float4 ce = a.bb_ext[cb];
+                const float dx = fmaxf(0.f, fabsf(wrap_delta(rc.x - cc.x, Lx, iLx)) - re.x - ce.x);
+                const float dy = fmaxf(0.f, fabsf(wrap_delta(rc.y - cc.y, Ly, iLy)) - re.y - ce.y);
+                const float dz = fmaxf(0.f, fabsf(wrap_delta(rc.z - cc.z, Lz, iLz)) - re.z - ce.z);
+                pass = dx * dx + dy * dy + dz * dz < r2;
             }
-            __syncthreads();
-            int queued = 0; // atoms in the warp's queue
-            for (int b0 = 0; b0 < windows * TB_WARPS; b0 += TILE) {
-                const unsigned mine =
-                    b0 + lane < windows * TB_WARPS ? sm.passing[b0 + lane] & (0x01010101u << warp) : 0u;
-                unsigned words = __ballot_sync(FULL_MASK, mine != 0);
-                int word = 0;
-                for (unsigned m = 0; m != 0 || words != 0; m &= m - 1) {
-                    if (m == 0) {
-                        word = __ffs(words) - 1;
-                        words &= words - 1;
-                        m = __shfl_sync(FULL_MASK, mine, word);
-                    }
-                    const int s = (c0 + (b0 + word) * TILE + __ffs(m) - 1) * TILE + lane;
-                    const bool valid = s < S;
-                    const float4 pj = valid ? a.posw[s] : make_float4(0.f, 0.f, 0.f, 0.f);
-                    // an atom farther than the radius from the row block's box is
-                    // farther than the radius from every row atom (widened test,
-                    // conservative under rounding): skip its per-row test
-                    const float wx = wrap_delta(pj.x - rc.x, Lx, iLx);
-                    const float wy = wrap_delta(pj.y - rc.y, Ly, iLy);
-                    const float wz = wrap_delta(pj.z - rc.z, Lz, iLz);
-                    const float bx = fmaxf(0.f, fabsf(wx) - re.x);
-                    const float by = fmaxf(0.f, fabsf(wy) - re.y);
-                    const float bz = fmaxf(0.f, fabsf(wz) - re.z);
-                    const bool need = valid && s >= col_lo && bx * bx + by * by + bz * bz < r2_box;
-                    // only the atoms in reach of the box (about half of a block)
-                    // go on to the row tests, 32 at a time
-                    const unsigned nmask = __ballot_sync(FULL_MASK, need);
-                    if (need) {
-                        sm.queue[warp][queued + __popc(nmask & lane_lt)] =
-                            make_float4(rc.x + wx, rc.y + wy, rc.z + wz, __int_as_float(s));
-                    }
-                    queued += __popc(nmask);
-                    if (queued >= TILE) {
-                        __syncwarp();
-                        tb_test_columns(sm, a, sm.queue[warp][lane], true, shifted, r2, Lx, Ly, Lz, iLx, iLy, iLz);
-                        queued -= TILE;
-                        const float4 rest = sm.queue[warp][TILE + lane];
-                        __syncwarp();
-                        sm.queue[warp][lane] = rest;
-                        __syncwarp();
-                    }
-                }
+            const unsigned m = __ballot_sync(FULL_MASK, pass);
+            if (lane == 0) {
+                sm.passing[i * TB_WARPS + warp] = m;
             }
-            __syncwarp();
-            if (queued > 0) {
-                tb_test_columns(sm, a, sm.queue[warp][lane], lane < queued, shifted, r2, Lx, Ly, Lz, iLx, iLy, iLz);
-            }
-            __syncthreads();
-            n_have = sm.n_cols;
-            __syncthreads(); // read by all before the next columns are added
-            if (!rounds && n_have > TB_COLS) {
-                break;
-            }
-            if (rounds && n_have + TB_ROUND * TILE > TB_COLS) {
-                tiles += tb_emit(sm, a, n_have, base_tile + tiles, false);
-                n_have = n_have % TILE;
-            }
-        }
-        if (n_have <= TB_COLS) {
-            break;
-        }
-        // more columns than the buffer holds: again, in rounds
-        if (threadIdx.x == 0) {
-            site_too_wide(a, row_first, state);
-        }
-        for (int k = threadIdx.x; k < TB_KEYS; k += TB_WARPS * 32) {
-            sm.bins[k] = 0;
-        }
-        if (threadIdx.x == 0) {
-            sm.n_cols = 0;
         }
         __syncthreads();
+        int queued = 0; // atoms in the warp's queue
+        for (int b0 = 0; b0 < windows * TB_WARPS; b0 += TILE) {
+            const unsigned mine =
+                b0 + lane < windows * TB_WARPS ? sm.passing[b0 + lane] & (0x01010101u << warp) : 0u;
+            unsigned words = __ballot_sync(FULL_MASK, mine != 0);
+            int word = 0;
+            for (unsigned m = 0; m != 0 || words != 0; m &= m - 1) {
+                if (m == 0) {
+                    word = __ffs(words) - 1;
+                    words &= words - 1;
+                    m = __shfl_sync(FULL_MASK, mine, word);
+                }
+                const int s = (c0 + (b0 + word) * TILE + __ffs(m) - 1) * TILE + lane;
+                const bool valid = s < S;
+                const float4 pj = valid ? a.posw[s] : make_float4(0.f, 0.f, 0.f, 0.f);
+                // an atom farther than the radius from the row block's box is
+                // farther than the radius from every row atom (widened test,
+                // conservative under rounding): skip its per-row test
+                const float wx = wrap_delta(pj.x - rc.x, Lx, iLx);
+                const float wy = wrap_delta(pj.y - rc.y, Ly, iLy);
+                const float wz = wrap_delta(pj.z - rc.z, Lz, iLz);
+                const float bx = fmaxf(0.f, fabsf(wx) - re.x);
+                const float by = fmaxf(0.f, fabsf(wy) - re.y);
+                const float bz = fmaxf(0.f, fabsf(wz) - re.z);
+                const bool need = valid && s >= col_lo && bx * bx + by * by + bz * bz < r2_box;
+                // only the atoms in reach of the box (about half of a block)
+                // go on to the row tests, 32 at a time
+                const unsigned nmask = __ballot_sync(FULL_MASK, need);
+                if (need) {
+                    sm.queue[warp][queued + __popc(nmask & lane_lt)] =
+                        make_float4(rc.x + wx, rc.y + wy, rc.z + wz, __int_as_float(s));
+                }
+                queued += __popc(nmask);
+                if (queued >= TILE) {
+                    __syncwarp();
+                    tb_test_columns(sm, a, sm.queue[warp][lane], true, shifted, r2, Lx, Ly, Lz, iLx, iLy, iLz, dst);
+                    queued -= TILE;
+                    const float4 rest = sm.queue[warp][TILE + lane];
+                    __syncwarp();
+                    sm.queue[warp][lane] = rest;
+                    __syncwarp();
+                }
+            }
+        }
+        __syncwarp();
+        if (queued > 0) {
+            tb_test_columns(sm, a, sm.queue[warp][lane], lane < queued, shifted, r2, Lx, Ly, Lz, iLx, iLy, iLz, dst);
+        }
+        __syncthreads(); // `passing` is written by the next pass, n_cols read below
     }
-    tiles += tb_emit(sm, a, n_have, base_tile + tiles, true);
+    const int tiles = tb_emit(sm, a, sm.n_cols, dst);
     if (warp == 0) {
         const int total = tiles;
         // the group's work items, at a range reserved from the list's

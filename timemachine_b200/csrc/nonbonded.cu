@@ -736,9 +736,10 @@ class NonbondedPotential : public PotentialBase {
         sa.n_site = (int)site_atoms_.n;
         // Many such atoms are worth the first slots to a multi-window call also where
         // their row groups are wide: 12 windows with a rebuild, plain order / first
-        // slots, 8,000 / 22,840 / 98,000 atoms: 1 % of the atoms, anywhere in the box,
-        // 167 / 172, 391 / 366, 1,509 / 1,736 us; 3 % 252 / 193, 640 / 430, 2,505 / 2,128.
-        sa.site_always = K > 1 && site_atoms_.n * 64 > (size_t)S_;
+        // slots, us: 1 % of 5,000 / 22,840 / 98,000 atoms anywhere in the box 127 / 101,
+        // 392 / 274, 1,509 / 1,371; 0.35 % of 22,840 (two ligands) 214 / 226, 0.2 %
+        // (a ligand and an ion) 203 / 227.
+        sa.site_always = K > 1 && site_atoms_.n * 128 > (size_t)S_;
         sa.grid_bits = grid_bits_;
         sa.hilbert = hilbert_ ? 1 : 0;
         sa.keys = keys_.p;

@@ -49,7 +49,7 @@ struct DevState {
     int dep_dirty;        // 1: the list of lambda-dependent tiles must be redone (rebuild, or lamdep changed)
     int items_chunk;      // tiles per work item in the list of the last rebuild
     int item_count;       // work items reserved so far by the rebuild in progress (0 between rebuilds)
-    int plain_order;      // rebuilds to come in which no site's atoms take the first slots (site_first)
+    int plain_until;      // rebuilds before this one keep the plain order (site_order)
 };
 
 // Error codes written into DevState::error (mirrored in include/tmnb.h).
@@ -358,10 +358,14 @@ __device__ __forceinline__ unsigned cell_key(const SortArgs &a, int atom) {
     return hilbert_index_3d(c[0], c[1], c[2], a.grid_bits);
 }
 
-// Whether this rebuild puts the site's atoms first; the same for every thread
-// (plain_order changes when the tile build is done).
+// Whether the site's atoms come first in this rebuild: not in the ones after a wide
+// row group. The same for every thread until the tile build has ended.
+__device__ __forceinline__ bool site_order(const DevState *state) {
+    const volatile DevState *now = state;
+    return now->rebuilds >= now->plain_until;
+}
 __device__ __forceinline__ bool site_first(const SortArgs &a, const DevState *state) {
-    return a.offset != nullptr && (a.site_always || *(const volatile int *)&state->plain_order == 0);
+    return a.offset != nullptr && (a.site_always || site_order(state));
 }
 // The cell at which the curve starts: next to the last site atom, so that the row
 // group which holds it is compact too.
@@ -933,8 +937,8 @@ __device__ __forceinline__ void build_tiles_cta(const TileArgs &a, const int rb,
             const float ex = mxx - mnx, ey = mxy - mny, ez = mxz - mnz;
             const float widest = 2.0f * SITE_EXTENT * a.cutoff;
             if (row_first < a.n_site && ex * ex + ey * ey + ez * ez > widest * widest &&
-                *(volatile int *)&state->plain_order == 0) {
-                state->plain_order = SITE_RETRY + 1; // one of them is this rebuild, taken off at its end
+                site_order(state)) {
+                state->plain_until = state->rebuilds + 1 + SITE_RETRY;
             }
         }
     }
@@ -1085,8 +1089,6 @@ __device__ __forceinline__ void build_tiles_cta(const TileArgs &a, const int rb,
         state->dep_dirty = 1; // the lambda-dependent tiles follow the new list
         state->n_dep = 0;
         state->rebuilds += 1;
-        const int plain = *(volatile int *)&state->plain_order;
-        state->plain_order = max(0, plain - 1);
         state->done_ctas = 0;
         state->rebuild = 0;
     }
